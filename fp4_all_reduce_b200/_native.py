@@ -1,9 +1,10 @@
-"""ctypes bindings of the two native libraries.
+"""Bindings of the native libraries.
 
 `oracle()` returns the host-only bit-exact model (always available: it is plain C++ and is built on
 first use).  `cuda()` returns the CUDA library; it is built in-tree by `python -m
 fp4_all_reduce_b200.build` and must exist on a GPU machine: the GPU ops raise instead of silently
-falling back to PyTorch when it is missing.
+falling back to PyTorch when it is missing.  `front()` returns the extension module that checks, allocates and
+launches one call of an op in C++, bound to the same CUDA library.
 """
 from __future__ import annotations
 
@@ -140,6 +141,25 @@ def cuda() -> C.CDLL:
                  "fp4ar_fill_sentinel"):
         getattr(lib, name).restype = C.c_int
     return lib
+
+
+@functools.lru_cache(maxsize=None)
+def front():
+    """The native front end (csrc/runtime/torch_front.cpp); also registers the CUDA kernels of `torch.ops.fp4ar`."""
+    import importlib.machinery
+    import importlib.util
+
+    path = _build.front_path()
+    if not path.exists():
+        raise RuntimeError(f"{path} is missing: build it with `python -m fp4_all_reduce_b200.build` (needs g++; no GPU required)")
+    import torch  # noqa: F401  (the module links against its libraries)
+
+    cuda()
+    loader = importlib.machinery.ExtensionFileLoader("_fp4ar_front", str(path))
+    mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_fp4ar_front", str(path), loader=loader))
+    loader.exec_module(mod)
+    mod.bind(str(cuda_library_path().resolve()), check)
+    return mod
 
 
 class ContextPoisoned(RuntimeError):

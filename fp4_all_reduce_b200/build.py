@@ -10,6 +10,7 @@ produces, next to this file,
 
     lib/libfp4ar.so         CUDA kernels + host runtime for sm_100a (nvcc, cross-compiles without a GPU)
     lib/libfp4ar_oracle.so  the host-only bit-exact model (g++)
+    lib/_fp4ar_front.so     the torch front end: checks, output allocation and launch of one call in C++ (g++, torch headers)
 
 Each translation unit is compiled separately and in parallel; an object is rebuilt when its source or
 any header under csrc/ changed.  ptxas resource usage of every kernel is appended to
@@ -131,6 +132,38 @@ def build_oracle(force: bool = False, verbose: bool = False) -> Path:
     return out
 
 
+def front_path() -> Path:
+    return LIB / "_fp4ar_front.so"
+
+
+def build_front(force: bool = False, verbose: bool = False) -> Path:
+    """The torch front end, an extension module of this interpreter against the installed torch's headers."""
+    import sysconfig
+
+    import torch
+
+    LIB.mkdir(exist_ok=True)
+    out = front_path()
+    src = CSRC / "runtime" / "torch_front.cpp"
+    t = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parent.parent
+    inc = [t / "include", t / "include" / "torch" / "csrc" / "api" / "include", cuda / "include", sysconfig.get_paths()["include"]]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[x for i in inc for x in ("-isystem", str(i))], str(src), "-o", str(out), f"-L{t / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu",
+           "-ltorch_cuda", "-ltorch_python"]
+    stamp_file = LIB / "front.stamp"
+    stamp = _stamp(src, _headers_digest() + torch.__version__ + sysconfig.get_python_version() + " ".join(cmd))
+    if not force and out.exists() and stamp_file.exists() and stamp_file.read_text() == stamp:
+        return out
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed:\n{r.stdout}\n{r.stderr}")
+    stamp_file.write_text(stamp)
+    if verbose:
+        print("[build] torch_front.cpp")
+    return out
+
+
 def check_compile(verbose: bool = False) -> int:
     """Compile every CUDA translation unit and the host model to objects; nothing is linked or installed."""
     OBJ.mkdir(exist_ok=True)
@@ -189,7 +222,10 @@ def resources(log: Path | None = None) -> list[dict]:
 
 
 def build_all(force: bool = False, verbose: bool = False) -> dict[str, Path]:
-    return {"oracle": build_oracle(force, verbose), "cuda": build_cuda(force, verbose)}
+    with cf.ThreadPoolExecutor(max_workers=1) as ex:
+        front = ex.submit(build_front, force, verbose)
+        libs = {"oracle": build_oracle(force, verbose), "cuda": build_cuda(force, verbose)}
+        return {**libs, "front": front.result()}
 
 
 def main(argv: list[str] | None = None) -> int:

@@ -213,6 +213,8 @@ decode_sum_kernel(SrcList src, long pitch, int rows, char* rec_out, char* out) {
         if (p == 0) {
           const uint32_t b = __float_as_uint(sc2.rs);
           *reinterpret_cast<uint4*>(r + kQRowBytes) = make_uint4(b, b, b, b);
+        } else if (p <= (kRecStride - kRecPayload) / 16) {   // the tail of the slot is zero: callers need not clear it
+          *reinterpret_cast<uint4*>(r + kRecPayload + 16 * (p - 1)) = make_uint4(0, 0, 0, 0);
         }
         zero32(acc);
         decode_acc_natural(acc, qq, sf2, sc2.rs);       // every rank outputs the decode of the re-encoding

@@ -33,6 +33,7 @@
 // with a copy (README.md:76, docs/INTEGRATION.md:67-74, harness/fp4ar_bench.cu:205-215).
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -677,7 +678,13 @@ static GemmPlan plan_gemm(int M, int N, int K, int sms, bool env) {
 template <int BN, int G>
 static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, cudaStream_t stream) {
   using S = GemmShape<BN, G>;
-  if (cudaFuncSetAttribute(gemm_nvfp4_kernel<BN, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem) != cudaSuccess) return cuda_fail();
+  // The shared-memory limit and the number of resident pairs are set / asked once per device, not on every launch.
+  static std::atomic<int> resident[64];          // 0: not asked yet; units (CTAs or pairs) that can be resident together
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cuda_fail();
+  int fits = resident[dev].load(std::memory_order_acquire);
+  if (!fits && cudaFuncSetAttribute(gemm_nvfp4_kernel<BN, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem) != cudaSuccess)
+    return cuda_fail();
   const int tiles = (p.N / BN) * ((p.M + kBM * G - 1) / (kBM * G));
   const int sms = device_sm_count();
   cudaLaunchConfig_t cfg;
@@ -693,10 +700,11 @@ static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams 
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.numAttrs = 1;
     cfg.gridDim = dim3(sms & ~1);
-    int clusters = 0;      // pairs that can be resident together: the grid is persistent, every pair must be
-    if (cudaOccupancyMaxActiveClusters(&clusters, gemm_nvfp4_kernel<BN, G>, &cfg) != cudaSuccess || clusters < 1) return cuda_fail();
-    if (clusters < units) units = clusters;
+    // pairs that can be resident together: the grid is persistent, every pair must be
+    if (!fits && (cudaOccupancyMaxActiveClusters(&fits, gemm_nvfp4_kernel<BN, G>, &cfg) != cudaSuccess || fits < 1)) return cuda_fail();
+    if (fits < units) units = fits;
   }
+  resident[dev].store(G == 2 ? fits : units, std::memory_order_release);     // every thread computes the same value
   // Programmatic dependent launch: a CTA may start (barrier set-up, TMEM allocation) on an SM that the previous
   // kernel's CTA has left while other CTAs of that kernel still run; it touches global memory only after
   // griddepcontrol.wait.  FP4AR_GEMM_PDL = 0 turns it off.

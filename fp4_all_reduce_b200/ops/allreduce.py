@@ -22,7 +22,6 @@ from typing import Dict
 import torch
 
 from .. import _native as N
-from . import codec as _codec
 
 _CONTEXTS: Dict[int, object] = {}
 _NEXT_ID = [1]
@@ -87,17 +86,6 @@ def _ar_norm_quant(x, residual, weight, eps, weight_bias, out_kind, qscale, ctx)
     return y
 
 
-def _add_rms_norm(x, residual, weight, eps, weight_bias):
-    y, _ = _codec.add_rmsnorm(x, residual, weight, eps, weight_bias, N.EPI_NORM_BF16, 1.0, inplace_residual=True)
-    return y
-
-
-def _linear_nvfp4(x, wt, gs):
-    from . import gemm as _gemm
-
-    return _gemm.gemm_nvfp4(x, wt, gs)
-
-
 def _linear_ar_norm(x, wt, gs, residual, weight, eps, weight_bias, ctx):
     from . import gemm as _gemm
 
@@ -110,12 +98,17 @@ _lib.impl("all_reduce_nvfp4", _all_reduce_nvfp4, "CUDA")
 _lib.impl("all_reduce_add_rms_norm", _ar_norm, "CUDA")
 _lib.impl("all_reduce_add_rms_norm_nvfp4", _ar_norm_nvfp4, "CUDA")
 _lib.impl("all_reduce_add_rms_norm_quant", _ar_norm_quant, "CUDA")
-_lib.impl("encode", lambda x: _codec.encode(x), "CUDA")
-_lib.impl("encode_static", lambda x, gs: _codec.encode_static(x, gs), "CUDA")
-_lib.impl("decode_sum", lambda q, r: _codec.decode_sum(list(q), list(r)), "CUDA")
-_lib.impl("add_rms_norm", _add_rms_norm, "CUDA")
-_lib.impl("linear_nvfp4", _linear_nvfp4, "CUDA")
 _lib.impl("linear_all_reduce_add_rms_norm", _linear_ar_norm, "CUDA")
+
+# The ops without a context have C++ kernels, registered when the front end is loaded.
+try:
+    N.front()
+except (RuntimeError, OSError, ImportError) as _e:          # not built here: the op says so when it is called
+    def _missing(*_args, _why=str(_e)):
+        raise RuntimeError(_why)
+
+    for _name in ("encode", "encode_static", "decode_sum", "add_rms_norm", "linear_nvfp4"):
+        _lib.impl(_name, _missing, "CUDA")
 
 
 def _bf16_rows(t):
