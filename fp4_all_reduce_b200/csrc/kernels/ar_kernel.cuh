@@ -21,9 +21,17 @@
 //     (slot k holds chunk k ^ ((lane >> 1) & 3)), so that every 64-byte-per-lane shared-memory access
 //     is bank-conflict free with static register indices; only the compact 16 B of E2M1 per pair is
 //     permuted, with 8 selects.
-//   * Input rows enter shared memory by bulk asynchronous copies; outputs and records leave through
-//     staging rows and one bulk store each.  The residual row of the norm epilogue goes global ->
-//     registers -> global (every lane owns whole 64-byte pieces).
+//   * Input and residual rows enter shared memory by bulk asynchronous copies through one ring of row
+//     buffers, each a whole step before it is used; outputs, the updated residual and records leave by one
+//     bulk store each.  (The residual used to go global -> registers -> global in 16-byte pieces at a
+//     64-byte stride, and its loads were issued where they were needed: finishing a row took 5000 - 6700
+//     cycles instead of 1250 without the epilogue.  16384 rows, BF16, one rank's work: two ranks 157 -> 145 us
+//     per block, four 198 -> 168, eight 232 -> 175 with the spills below gone; 123 us at the copy rate.)
+//   * Registers bound the six-warp shapes (96 a thread, 18 warps): what spills does not fit the L1 that the
+//     shared memory leaves, and a 12-byte spill in the loop costs 5 - 10 %.  Hence the owner step takes its
+//     sources in batches and addresses are recomputed instead of kept.
+//   * Calls of one or two rows per CTA have a narrow build (MT teams at most, six warps each, up to 168
+//     registers): they are one row's latency, see the rule in runtime.cu.
 //   * Every wait is bounded (see fp4ar_async.cuh).
 #pragma once
 #include "../include/fp4ar_codec.cuh"
@@ -56,13 +64,15 @@ struct ArParams {
   float gs[kMaxRanks];
   float eps, wbias, qscale;
   int rows, ctas_per_rank, flags;
+  int rows_q, rows_r;                 // rows / ctas_per_rank and the remainder
   int cap, capo;
   unsigned long long buf_bytes, timeout_ns;
+  unsigned long long rs_stride;       // capo slots: from one source's two-shot slots to the next one's
   int lag_owner, lag_finish;          // two-shot pipeline depths in steps (1 <= lag_owner < lag_finish <= 4)
   unsigned long long* phase_cycles;   // tuning builds only (-DFP4AR_PHASE_TIMERS): 16 per-phase cycle counters
 };
 
-template <int P, int ALGO, int IN, int EPI, int T>
+template <int P, int ALGO, int IN, int EPI, int T, int MT = 0>
 struct ArShape {
   static constexpr int NJ = 6 / T;                                   // pairs per lane per row
   static constexpr bool kTwoShot = ALGO == 1 && P > 1;
@@ -72,11 +82,13 @@ struct ArShape {
   // The two-shot lags are run-time parameters (owner step lag_o >= 1 steps after the encode, finish lag_f > lag_o);
   // kMaxLag bounds them and sizes the record ring.
   static constexpr int kMaxLag = kTwoShot ? 4 : 1;
-  static constexpr int NXB = IN == 0 ? 2 : 0;                        // x row buffers (the residual never sits in shared memory)
+  // Row buffers, a ring over the rows in the order in which a team consumes them: x of step k, residual of step k, x of
+  // step k + 1, ...  Each is loaded a whole step before it is used.
+  static constexpr int NRB = IN == 0 ? (EPI > 0 ? 3 : 2) : (EPI > 0 ? 2 : 0);
   static constexpr int NREC = (IN == 1 ? 2 : 1) + kMaxLag;
   static constexpr int kOutBytes = EPI <= 1 ? kRowBytes : (EPI == 2 ? 3584 : 6400);
   static constexpr int kMisc = 128;                                  // mbarriers + reduction scratch
-  static constexpr int kTeamBytes = NXB * kRowBytes + kOutBytes + NREC * kRecStride + kMisc;
+  static constexpr int kTeamBytes = NRB * kRowBytes + kOutBytes + NREC * kRecStride + kMisc;
   static constexpr int kCtaExtra = kRecStride + 128 + 1024;          // sentinel record + abort flag + scale table
   static constexpr int NSG = IN == 2 ? P : P - 1;                    // sources read from the window
   // Two-shot owners hold a whole FP32 row slice in registers and the norm epilogue holds BF16 z and the
@@ -85,7 +97,7 @@ struct ArShape {
   static constexpr int kHeavy = (ALGO == 1 || EPI > 0) ? 1 : 0;
   // Three-warp teams: 4 per CTA (heavy shapes) or 5; six-warp teams: 3 per CTA (18 warps at up to 112 registers; a
   // fourth team at 80 registers measured 20-30 % slower).
-  static constexpr int kMaxTeams = T == 3 ? (kHeavy ? 4 : 5) : (T == 1 ? 8 : 3);
+  static constexpr int kMaxTeams = MT > 0 ? MT : (T == 3 ? (kHeavy ? 4 : 5) : 3);
   static __host__ __device__ constexpr int smem_bytes(int teams) { return teams * kTeamBytes + kCtaExtra; }
 };
 
@@ -143,12 +155,12 @@ struct TeamSync {
   }
 };
 
-template <int P, int ALGO, int IN, int EPI, int T>
-__global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T>::kMaxTeams, 1) ar_kernel(const __grid_constant__ ArParams prm) {
-  using S = ArShape<P, ALGO, IN, EPI, T>;
-  constexpr int NJ = S::NJ, NXB = S::NXB, NREC = S::NREC, NSG = S::NSG;
+template <int P, int ALGO, int IN, int EPI, int T, int MT>
+__global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T, MT>::kMaxTeams, 1) ar_kernel(const __grid_constant__ ArParams prm) {
+  using S = ArShape<P, ALGO, IN, EPI, T, MT>;
+  constexpr int NJ = S::NJ, NREC = S::NREC, NSG = S::NSG;
   constexpr bool kTwoShot = S::kTwoShot;
-  constexpr int NXB1 = NXB > 0 ? NXB : 1;   // keeps index arithmetic well-formed in shapes without row buffers
+  constexpr int NRB1 = S::NRB > 0 ? S::NRB : 1;   // keeps index arithmetic well-formed in shapes without row buffers
   extern __shared__ __align__(1024) uint8_t smem[];
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -165,11 +177,11 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T>::kMaxTea
 
   // ---- shared-memory carve-up ----
   uint8_t* tbase = smem + (size_t)team * S::kTeamBytes;
-  uint8_t* xb = tbase;                                   // NXB buffers for BF16 input rows
-  uint8_t* outst = tbase + NXB * kRowBytes;              // output staging row
+  uint8_t* rowb = tbase;                                 // NRB row buffers
+  uint8_t* outst = rowb + S::NRB * kRowBytes;            // output staging row
   uint8_t* recs = outst + S::kOutBytes;                  // NREC encoded records
-  uint64_t* xbar = reinterpret_cast<uint64_t*>(recs + NREC * kRecStride);  // [3] x loads
-  uint64_t* qbar = xbar + 2;                             // [6] NVFP4 record loads
+  uint64_t* rowbar = reinterpret_cast<uint64_t*>(recs + NREC * kRecStride);  // [3] row loads
+  uint64_t* qbar = rowbar + 3;                           // [6] NVFP4 record loads
   float* red = reinterpret_cast<float*>(qbar + 6);       // [2][6] reduction exchange
   uint8_t* sentinel = smem + (size_t)nteams * S::kTeamBytes;
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(sentinel + kRecStride);
@@ -181,7 +193,7 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T>::kMaxTea
   if (threadIdx.x == 0) *abort_flag = 0u;
   if (leader) {
 #pragma unroll
-    for (int i = 0; i < 8; i++) mbar_init(xbar + i, 1);
+    for (int i = 0; i < 9; i++) mbar_init(rowbar + i, 1);
   }
   for (int i = threadIdx.x; i < kRecStride / 16; i += blockDim.x) {
     uint4 v;
@@ -195,19 +207,24 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T>::kMaxTea
   mbar_init_fence();
   fence_smem_to_async();
   __syncthreads();
-  const int rb = (int)(((long long)cta * prm.rows) / G), re = (int)(((long long)(cta + 1) * prm.rows) / G);
+  // contiguous rows per CTA, the first rows_r of them one row longer (quotient and remainder from the host)
+  const int rb = cta * prm.rows_q + min(cta, prm.rows_r), re = rb + prm.rows_q + (cta < prm.rows_r ? 1 : 0);
   const int nk = (re - rb > team) ? (re - rb - team + nteams - 1) / nteams : 0;
   auto row_of = [&](int k) { return rb + team + nteams * k; };
+  // Items of the row ring: x of step k and the residual of the row finished in step k.
+  auto x_item = [](int k) { return EPI > 0 ? 2 * k : k; };
+  auto res_item = [](int k) { return IN == 0 ? 2 * k + 1 : k; };
+  auto load_row = [&](int item, const char* base, int row) {
+    const int b = item % NRB1;
+    mbar_arrive_expect(rowbar + b, kRowBytes);
+    bulk_load(rowb + b * kRowBytes, base + (size_t)row * kRowBytes, kRowBytes, rowbar + b);
+  };
   pdl_wait_prior_grids();
   // ---- first loads: they need nothing from the call state, so they go out before it is read ----
   if (leader && nk > 0) {
     if (IN == 0) {
-      mbar_arrive_expect(xbar + 0, kRowBytes);
-      bulk_load(xb, io.x + (size_t)row_of(0) * kRowBytes, kRowBytes, xbar + 0);
-      if (nk > 1) {
-        mbar_arrive_expect(xbar + 1, kRowBytes);
-        bulk_load(xb + kRowBytes, io.x + (size_t)row_of(1) * kRowBytes, kRowBytes, xbar + 1);
-      }
+      load_row(x_item(0), io.x, row_of(0));
+      if (nk > 1) load_row(x_item(1), io.x, row_of(1));
     } else if (IN == 1) {
       mbar_arrive_expect(qbar + 0, kQRowBytes);
       bulk_load(recs, io.x + (size_t)row_of(0) * kQRowBytes, kQRowBytes, qbar + 0);
@@ -221,12 +238,23 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T>::kMaxTea
   wctx.status = io.status; wctx.cta_abort = abort_flag; wctx.host_poison = io.poison; wctx.limit_ns = prm.timeout_ns;
   wctx.cta = (uint32_t)cta; wctx.call = call;
 
-  const size_t buf_off = (size_t)(call & 1u) * prm.buf_bytes;
-  char* const my_buf = io.win[me] + buf_off;
+  // Recomputed from the parity where they are used: registers kept around the whole loop are what makes the six-warp
+  // shapes spill, and spills do not fit the L1 that the shared memory leaves (a 12-byte spill cost 5 - 10 %).
+  const uint32_t parity = call & 1u;
+  auto buf_off = [&]() -> size_t { return parity ? prm.buf_bytes : 0; };
+  auto my_buf = [&]() -> char* { return io.win[me] + buf_off(); };
   const int cap = prm.cap, capo = prm.capo;
   auto os_slot = [&](int src, int row) -> size_t { return ((size_t)src * cap + row) * kRecStride; };
   auto rs_slot = [&](int src, int row) -> size_t { return ((size_t)src * capo + row / P) * kRecStride; };
   auto ag_slot = [&](int own, int row) -> size_t { return ((size_t)(P + own) * capo + row / P) * kRecStride; };
+
+  uint32_t row_phase = 0;                       // parity of every ring buffer's next load
+  auto wait_row = [&](int item, int row) -> uint8_t* {
+    const int b = item % NRB1;
+    mbar_wait_bounded(rowbar + b, (row_phase >> b) & 1u, wctx, (uint32_t)row);
+    row_phase ^= 1u << b;
+    return rowb + b * kRowBytes;
+  };
 
   int red_phase = 0;
 
@@ -248,7 +276,7 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T>::kMaxTea
   // order; this routine applies the epilogue, stages the row and lets the leader store it.
   // `leader_extra()` issues the leader's other stores of this row (re-arm, broadcast).
   // =============================================================================================
-  auto finish_row = [&](int row, auto&& fill, auto&& leader_extra) {
+  auto finish_row = [&](int row, int step, auto&& fill, auto&& leader_extra) {
     const int pbase = tw;  // pair of (lane, j) = lane + 32 * (tw + T * j)
     if constexpr (EPI == 0) {
 #pragma unroll
@@ -268,18 +296,9 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T>::kMaxTea
         leader_extra();
       }
     } else {
-      // The residual row is read straight from global memory into registers (issued before the window data is
-      // polled and decoded, so its latency is hidden) and the updated residual is written straight back: each lane
-      // touches whole 64-byte pieces, so every 32-byte sector it reads or writes is fully used.
-      const char* res_row = io.res_in + (size_t)row * kRowBytes;
-      char* res_out_row = io.res_out + (size_t)row * kRowBytes;
-      uint4 rr[NJ][4];
-#pragma unroll
-      for (int j = 0; j < NJ; j++) {
-        const int p = lane + 32 * (pbase + T * j);
-#pragma unroll
-        for (int k = 0; k < 4; k++) rr[j][k] = *reinterpret_cast<const uint4*>(res_row + p * 64 + ((k ^ f) << 4));
-      }
+      // The residual row was brought into its ring buffer by a bulk load a step ago; z = BF16(sum + residual) replaces
+      // it there and leaves by a bulk store.
+      uint8_t* resb = wait_row(res_item(step), row);
       uint4 zb[NJ][4];
       float gsum[NJ];
 #pragma unroll
@@ -287,15 +306,29 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T>::kMaxTea
         const int p = lane + 32 * (pbase + T * j);
         float acc[32];
         fill(j, acc);
-        const float sp = add_residual_sumsq(acc, rr[j]);
+        uint4 rr[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) rr[k] = lds16(resb + p * 64 + ((k ^ f) << 4));
+        const float sp = add_residual_sumsq(acc, rr);
         pack32_bf16(acc, zb[j]);
 #pragma unroll
-        for (int k = 0; k < 4; k++) *reinterpret_cast<uint4*>(res_out_row + p * 64 + ((k ^ f) << 4)) = zb[j][k];
+        for (int k = 0; k < 4; k++) sts16(resb + p * 64 + ((k ^ f) << 4), zb[j][k]);
         gsum[j] = warp_sum_butterfly(sp);
+      }
+      fence_smem_to_async();
+      uint4 wt[NJ][4];          // fetched across the exchange
+#pragma unroll
+      for (int j = 0; j < NJ; j++) {
+        const int p = lane + 32 * (pbase + T * j);
+#pragma unroll
+        for (int k = 0; k < 4; k++) wt[j][k] = __ldg(reinterpret_cast<const uint4*>(prm.weight + p * 64 + ((k ^ f) << 4)));
       }
       float g6[6];
       team_gather6(gsum, g6);   // also: every lane is done polling, so the slots may be re-armed
-      if (leader) leader_extra();
+      if (leader) {
+        bulk_store(io.res_out + (size_t)row * kRowBytes, resb, kRowBytes);
+        leader_extra();
+      }
       float ss = g6[0];
 #pragma unroll
       for (int g = 1; g < 6; g++) ss = __fadd_rn(ss, g6[g]);
@@ -303,11 +336,8 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T>::kMaxTea
 #pragma unroll
       for (int j = 0; j < NJ; j++) {
         const int p = lane + 32 * (pbase + T * j);
-        uint4 wt[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) wt[k] = __ldg(reinterpret_cast<const uint4*>(prm.weight + p * 64 + ((k ^ f) << 4)));
         float y[32];
-        norm_pair(zb[j], wt, rinv, prm.wbias, y);
+        norm_pair(zb[j], wt[j], rinv, prm.wbias, y);
         uint4 yb[4];
         pack32_bf16(y, yb);
         if (EPI == 1) {
@@ -395,60 +425,22 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T>::kMaxTea
   const int lag_f = kTwoShot ? prm.lag_finish : 1;
   for (int k = 0; k < nk + lag_f; k++) {
     FP4AR_PHASE(0);
-    if (leader) bulk_wait_source_free<0>();
+    if (kTwoShot ? lane == 0 : leader) bulk_wait_source_free<0>();
     tsync.sync();
     FP4AR_PHASE(1);   // drain wait + barrier
+    if (EPI > 0 && leader) {                    // the buffer of the residual that left in the previous step is free
+      if (IN == 0) {
+        if (k > 0 && k + 1 < nk) load_row(x_item(k + 1), io.x, row_of(k + 1));
+      } else {
+        const int kr = k + 1 - lag_f;
+        if (kr >= 0 && kr < nk) load_row(res_item(k + 1), io.res_in, row_of(kr));
+      }
+    }
     if (leader && IN == 1 && k + 1 < nk) {
       const int b = (k + 1) % NREC;
       mbar_arrive_expect(qbar + b, kQRowBytes);
       bulk_load(recs + b * kRecStride, io.x + (size_t)row_of(k + 1) * kQRowBytes, kQRowBytes, qbar + b);
     }
-
-    // ------------------------------------------------------------------ early window loads
-    // (a) the row finished in this step (k - lag_f): one-shot sources, or the owner's broadcast of a row owned by a peer;
-    // (b) two-shot: the reduce-scatter sources of row k - lag_owner when this rank owns it (loaded in the owner step).
-    // Everything was pushed at least one full step ago; stage-specific code validates and falls back to polling.
-    const int kf = k - lag_f;                        // row index (in this team's sequence) finished in this step
-    const bool fin = kf >= 0 && kf < nk;
-    const int frow = fin ? row_of(kf) : 0;
-    const bool fin_owned = kTwoShot && fin && (frow % P) == me;
-    const char* fsrc[kTwoShot ? 1 : kPfSrc];
-    uint32_t frs[kTwoShot ? 1 : kPfSrc];
-    uint4 fq[NJ][kTwoShot ? 1 : (kPfAll ? kPfSrc : 1)];
-    uint32_t fsf[NJ][kTwoShot ? 1 : (kPfAll ? kPfSrc : 1)];
-    bool f_has_rs = false;
-    if (fin) {
-      if constexpr (!kTwoShot) {
-#pragma unroll
-        for (int i = 0; i < NSG; i++) fsrc[i] = my_buf + os_slot(window_source(i), frow);
-        f_has_rs = IN == 0;
-#pragma unroll
-        for (int i = 0; i < NSG; i++)
-          if (f_has_rs) frs[i] = poll_ld4(fsrc[i] + kQRowBytes);
-        if (kPfAll) {
-#pragma unroll
-          for (int jj = 0; jj < NJ; jj++) {
-            const int p = lane + 32 * (tw + T * jj);
-#pragma unroll
-            for (int i = 0; i < NSG; i++) {
-              fq[jj][i] = poll_ld16(fsrc[i] + 16 * p);
-              fsf[jj][i] = poll_ld2(fsrc[i] + kValueBytes + 2 * p);
-            }
-          }
-        }
-      } else if (!fin_owned) {
-        fsrc[0] = my_buf + ag_slot(frow % P, frow);
-        f_has_rs = !(loopb && IN >= 1);
-        if (f_has_rs) frs[0] = poll_ld4(fsrc[0] + kQRowBytes);
-#pragma unroll
-        for (int jj = 0; jj < NJ; jj++) {
-          const int p = lane + 32 * (tw + T * jj);
-          fq[jj][0] = poll_ld16(fsrc[0] + 16 * p);
-          fsf[jj][0] = poll_ld2(fsrc[0] + kValueBytes + 2 * p);
-        }
-      }
-    }
-    FP4AR_PHASE(2);   // early loads issued
 
     // ------------------------------------------------------------------ owner step of row k-lag_o (two-shot)
     // Reduce every source, re-encode into rec, broadcast.  The row is finished (decoded, epilogue) lag_finish -
@@ -458,63 +450,98 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T>::kMaxTea
       if (ko >= 0 && ko < nk && (row_of(ko) % P) == me) {
         const int row = row_of(ko);
         uint8_t* rec_own = recs + (ko % NREC) * kRecStride;
-        const char* osrc[kPfSrc];
-        float wrs[kPfSrc];
-        uint32_t ors[kPfSrc];
-#pragma unroll
-        for (int i = 0; i < NSG; i++) {
-          osrc[i] = my_buf + rs_slot(window_source(i), row);
-          if (IN == 0) ors[i] = poll_ld4(osrc[i] + kQRowBytes);
-        }
-        uint4 oq[NJ][kPfAll ? kPfSrc : 1];
-        uint32_t osf[NJ][kPfAll ? kPfSrc : 1];
-        if (kPfAll) {
-#pragma unroll
-          for (int jj = 0; jj < NJ; jj++) {
-            const int p = lane + 32 * (tw + T * jj);
-#pragma unroll
-            for (int i = 0; i < NSG; i++) {
-              oq[jj][i] = poll_ld16(osrc[i] + 16 * p);
-              osf[jj][i] = poll_ld2(osrc[i] + kValueBytes + 2 * p);
-            }
+        // Every rank's contribution in rank order, kOwnBatch ranks at a time: the loads of a batch are issued together,
+        // and where some have not arrived all of those are asked for again
+        // together, one round trip for all instead of one each.  The own contribution comes from the record ring.
+        constexpr int kOwnBatch = MT > 0 ? P : (P == 4 ? 4 : 2);
+        char* const src0 = my_buf() + rs_slot(0, row);
+        auto own_src = [&](int src) { return src0 + (size_t)src * prm.rs_stride; };
+        auto own_load = [&](int src, int p, uint4& q, uint32_t& sf, uint32_t& rsb) {
+          if (IN != 2 && src == me) {
+            q = lds16(rec_own + 16 * p);
+            sf = *reinterpret_cast<const uint16_t*>(rec_own + kValueBytes + 2 * p);
+            rsb = IN == 0 ? *reinterpret_cast<const uint32_t*>(rec_own + kQRowBytes) : __float_as_uint(prm.gs[src]);
+          } else {
+            const char* c = own_src(src);
+            q = poll_ld16(c + 16 * p);
+            sf = poll_ld2(c + kValueBytes + 2 * p);
+            rsb = IN == 0 ? poll_ld4(c + kQRowBytes) : __float_as_uint(prm.gs[src]);
           }
-        }
-#pragma unroll
-        for (int i = 0; i < NSG; i++) {
-          const int s = window_source(i);
-          wrs[i] = IN == 0 ? settle_rs(ors[i], osrc[i], row, s, 2) : prm.gs[s];
-        }
-        float own_rs = 0.0f;
-        if (IN == 0) own_rs = *reinterpret_cast<const float*>(rec_own + kQRowBytes);
-        if (IN == 1) own_rs = prm.gs[me];
+        };
+        auto own_pending = [&](uint4 q, uint32_t sf, uint32_t rsb) {
+          return values_pending(q) | scales_pending(sf) | (IN == 0 && rowscale_pending(rsb));
+        };
         float sums[NJ][32];
         float am = 0.0f;
 #pragma unroll
         for (int j = 0; j < NJ; j++) {
           const int p = lane + 32 * (tw + T * j);
-          uint4 wq[kPfSrc];
-          uint32_t wsf[kPfSrc];
-#pragma unroll
-          for (int i = 0; i < NSG; i++) {
-            if (kPfAll) { wq[i] = oq[j][i]; wsf[i] = osf[j][i]; }
-            else { wq[i] = poll_ld16(osrc[i] + 16 * p); wsf[i] = poll_ld2(osrc[i] + kValueBytes + 2 * p); }
-          }
-#pragma unroll
-          for (int i = 0; i < NSG; i++)
-            if (values_pending(wq[i]) | scales_pending(wsf[i])) poll_pair(osrc[i], p, wq[i], wsf[i], row, window_source(i), 2);
           zero32(sums[j]);
-          if (!xport) {
+#pragma unroll 1
+          for (int s0 = 0; s0 < P; s0 += kOwnBatch) {
+            uint4 wq[kOwnBatch];
+            uint32_t wsf[kOwnBatch], wrs[kOwnBatch];
 #pragma unroll
-            for (int i = 0; i <= NSG; i++) {
-              if (IN != 2 && i == me) {
-                const uint4 q = lds16(rec_own + 16 * p);
-                const uint32_t sf2 = *reinterpret_cast<const uint16_t*>(rec_own + kValueBytes + 2 * p);
-                decode_acc_lane(sums[j], q, sf2, own_rs, f);
+            for (int u = 0; u < kOwnBatch; u++) own_load(s0 + u, p, wq[u], wsf[u], wrs[u]);
+            bool pend = false;
+#pragma unroll
+            for (int u = 0; u < kOwnBatch; u++) pend |= own_pending(wq[u], wsf[u], wrs[u]);
+            if (MT == 0 && pend) {
+              const unsigned long long t0 = global_timer_ns();
+              uint32_t n = 0;
+              while (!*abort_flag) {
+                uint32_t missing = 0;
+#pragma unroll
+                for (int u = 0; u < kOwnBatch; u++)
+                  if (own_pending(wq[u], wsf[u], wrs[u])) { own_load(s0 + u, p, wq[u], wsf[u], wrs[u]); missing = u; }
+                pend = false;
+#pragma unroll
+                for (int u = 0; u < kOwnBatch; u++) pend |= own_pending(wq[u], wsf[u], wrs[u]);
+                if (!pend) break;
+                if ((++n & 127u) == 0u && global_timer_ns() - t0 > prm.timeout_ns) {
+                  report_wait_failure(wctx, kStatusPeerTimeout, (uint32_t)row, (uint32_t)s0 + missing, 2u);
+                  break;
+                }
               }
-              if (i < NSG) decode_acc_lane(sums[j], wq[i], wsf[i], wrs[i], f);
             }
-            am = absmax32(sums[j], am);
+            if (MT > 0 && __any_sync(0xffffffffu, pend)) {
+              // One lane per source watches the last scale pair of its record, which costs a load per round instead of
+              // three per source and lane; then everything that was missing is loaded again.
+              const unsigned long long t0 = global_timer_ns();
+              uint32_t n = 0;
+              while (true) {             // every decision is the whole warp's
+                if (__any_sync(0xffffffffu, *abort_flag != 0u)) break;
+                const int src = s0 + lane;
+                bool miss = lane < kOwnBatch && (IN == 2 || src != me) &&
+                            scales_pending(poll_ld2(own_src(src) + kValueBytes + kScaleBytes - 2));
+                if (!__any_sync(0xffffffffu, miss)) {
+#pragma unroll
+                  for (int u = 0; u < kOwnBatch; u++)
+                    if (own_pending(wq[u], wsf[u], wrs[u])) own_load(s0 + u, p, wq[u], wsf[u], wrs[u]);
+                  pend = false;
+#pragma unroll
+                  for (int u = 0; u < kOwnBatch; u++) {
+                    const bool still = own_pending(wq[u], wsf[u], wrs[u]);
+                    pend |= still;
+                    if (__any_sync(0xffffffffu, still)) miss |= lane == u;
+                  }
+                  if (!__any_sync(0xffffffffu, pend)) break;
+                }
+                const bool late = (++n & 127u) == 0u && global_timer_ns() - t0 > prm.timeout_ns;
+                if (__any_sync(0xffffffffu, late)) {
+                  const uint32_t which = __ballot_sync(0xffffffffu, miss);
+                  if (lane == 0)
+                    report_wait_failure(wctx, kStatusPeerTimeout, (uint32_t)row, (uint32_t)(s0 + (which ? __ffs((int)which) - 1 : 0)), 2u);
+                  break;
+                }
+              }
+            }
+            if (!xport) {
+#pragma unroll
+              for (int u = 0; u < kOwnBatch; u++) decode_acc_lane(sums[j], wq[u], wsf[u], __uint_as_float(wrs[u]), f);
+            }
           }
+          if (!xport) am = absmax32(sums[j], am);
         }
         am = warp_max(am);
         {
@@ -557,28 +584,71 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T>::kMaxTea
         }
         fence_smem_to_async();
         tsync.sync();
-        if (leader) {
-#pragma unroll
-          for (int d = 0; d < P; d++) {
-            if (d == me) continue;
-            char* dst = (loopb ? my_buf : io.win[d] + buf_off) + ag_slot(me, row);
-            bulk_store(dst, rec_own, kRecPayload);
+        // broadcast and re-arm, the peers shared out over the team's warps (not unrolled: the addresses would be kept in
+        // registers around the whole loop)
+        if (lane == 0) {
+#pragma unroll 1
+          for (int d = tw; d < P; d += T) {
+            if (d != me) bulk_store((loopb ? my_buf() : io.win[d] + buf_off()) + ag_slot(me, row), rec_own, kRecPayload);
+            if (IN == 2 || d != me) bulk_store(own_src(d), sentinel, kRecPayload);
           }
-#pragma unroll
-          for (int i = 0; i < NSG; i++) bulk_store(const_cast<char*>(osrc[i]), sentinel, kRecPayload);
         }
       }
     }
     FP4AR_PHASE(3);   // owner step
+
+    // ------------------------------------------------------------------ early window loads
+    // The row finished in this step (k - lag_f): one-shot sources, or the owner's broadcast of a row owned by a peer;
+    // (the reduce-scatter sources of an owned row are loaded in the owner step above).
+    // Everything was pushed at least one full step ago; stage-specific code validates and falls back to polling.
+    const int kf = k - lag_f;                        // row index (in this team's sequence) finished in this step
+    const bool fin = kf >= 0 && kf < nk;
+    const int frow = fin ? row_of(kf) : 0;
+    const bool fin_owned = kTwoShot && fin && (frow % P) == me;
+    const char* fsrc[kTwoShot ? 1 : kPfSrc];
+    uint32_t frs[kTwoShot ? 1 : kPfSrc];
+    uint4 fq[NJ][kTwoShot ? 1 : (kPfAll ? kPfSrc : 1)];
+    uint32_t fsf[NJ][kTwoShot ? 1 : (kPfAll ? kPfSrc : 1)];
+    bool f_has_rs = false;
+    if (fin) {
+      if constexpr (!kTwoShot) {
+#pragma unroll
+        for (int i = 0; i < NSG; i++) fsrc[i] = my_buf() + os_slot(window_source(i), frow);
+        f_has_rs = IN == 0;
+#pragma unroll
+        for (int i = 0; i < NSG; i++)
+          if (f_has_rs) frs[i] = poll_ld4(fsrc[i] + kQRowBytes);
+        if (kPfAll) {
+#pragma unroll
+          for (int jj = 0; jj < NJ; jj++) {
+            const int p = lane + 32 * (tw + T * jj);
+#pragma unroll
+            for (int i = 0; i < NSG; i++) {
+              fq[jj][i] = poll_ld16(fsrc[i] + 16 * p);
+              fsf[jj][i] = poll_ld2(fsrc[i] + kValueBytes + 2 * p);
+            }
+          }
+        }
+      } else if (!fin_owned) {
+        fsrc[0] = my_buf() + ag_slot(frow % P, frow);
+        f_has_rs = !(loopb && IN >= 1);
+        if (f_has_rs) frs[0] = poll_ld4(fsrc[0] + kQRowBytes);
+#pragma unroll
+        for (int jj = 0; jj < NJ; jj++) {
+          const int p = lane + 32 * (tw + T * jj);
+          fq[jj][0] = poll_ld16(fsrc[0] + 16 * p);
+          fsf[jj][0] = poll_ld2(fsrc[0] + kValueBytes + 2 * p);
+        }
+      }
+    }
+    FP4AR_PHASE(2);   // early loads issued
 
     // ------------------------------------------------------------------ stage A: encode + push row k
     if (k < nk) {
       const int row = row_of(k);
       uint8_t* rec = recs + (k % NREC) * kRecStride;
       if (IN == 0) {
-        const int b = k % NXB1;
-        const uint8_t* xrow = xb + b * kRowBytes;
-        mbar_wait_bounded(xbar + b, (uint32_t)((k / NXB1) & 1), wctx, row);
+        const uint8_t* xrow = wait_row(x_item(k), row);
         FP4AR_PHASE(4);   // wait for x
         if (!xport) {
           uint32_t bmp[NJ];
@@ -650,27 +720,28 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T>::kMaxTea
 #pragma unroll
             for (int d = 0; d < P; d++) {
               if (d == me) continue;
-              char* dst = loopb ? my_buf + os_slot(d, row) : io.win[d] + buf_off + os_slot(me, row);
+              char* dst = loopb ? my_buf() + os_slot(d, row) : io.win[d] + buf_off() + os_slot(me, row);
               bulk_store(dst, rec, bytes);
             }
           } else {
             const int owner = row % P;
             if (owner != me) {
-              char* dst = loopb ? my_buf + ag_slot(owner, row) : io.win[owner] + buf_off + rs_slot(me, row);
+              char* dst = loopb ? my_buf() + ag_slot(owner, row) : io.win[owner] + buf_off() + rs_slot(me, row);
               bulk_store(dst, rec, bytes);
-            } else if (loopb) {
-#pragma unroll
-              for (int s = 0; s < P; s++)
-                if (s != me) bulk_store(my_buf + rs_slot(s, row), rec, bytes);
             }
           }
         }
-        if (IN == 0 && k + 2 < nk) {
-          const int b = k % NXB1;
-          mbar_arrive_expect(xbar + b, kRowBytes);
-          bulk_load(xb + b * kRowBytes, io.x + (size_t)row_of(k + 2) * kRowBytes, kRowBytes, xbar + b);
-        }
+        if (IN == 0 && EPI == 0 && k + 2 < nk) load_row(x_item(k + 2), io.x, row_of(k + 2));
       }
+    }
+    if (kTwoShot && IN != 2 && loopb && lane == 0 && k < nk && row_of(k) % P == me) {     // compute mode: the peers' contributions
+#pragma unroll 1
+      for (int s = tw; s < P; s += T)
+        if (s != me) bulk_store(my_buf() + rs_slot(s, row_of(k)), recs + (k % NREC) * kRecStride, IN == 0 ? (uint32_t)kRecPayload : (uint32_t)kQRowBytes);
+    }
+    if (IN == 0 && EPI > 0 && leader) {         // into the buffer of the row just encoded
+      const int kr = k + 1 - lag_f;
+      if (kr >= 0 && kr < nk) load_row(res_item(k + 1), io.res_in, row_of(kr));
     }
     FP4AR_PHASE(6);   // encode pass 2 + push
 
@@ -718,7 +789,7 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T>::kMaxTea
 #pragma unroll
           for (int i = 0; i < NSG; i++) bulk_store(const_cast<char*>(fsrc[i]), sentinel, kRecPayload);
         };
-        finish_row(row, fill, extra);
+        finish_row(row, k, fill, extra);
       } else {
         if (fin_owned) {
           // ---- two-shot, owned row: its re-encoding sits in the ring; every rank outputs the decode of that ----
@@ -733,7 +804,7 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T>::kMaxTea
             }
           };
           auto extra = [&]() {};
-          finish_row(row, fill, extra);
+          finish_row(row, k, fill, extra);
         } else {
           // ---- two-shot, row owned by a peer: its broadcast had lag_finish - lag_owner steps to arrive ----
           const char* src = fsrc[0];
@@ -748,15 +819,15 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T>::kMaxTea
             if (!xport) decode_acc_lane(acc, wq, wsf, rs, f);
           };
           auto extra = [&]() { bulk_store(const_cast<char*>(src), sentinel, kRecPayload); };
-          finish_row(row, fill, extra);
+          finish_row(row, k, fill, extra);
         }
       }
     }
     FP4AR_PHASE(7);   // finish
-    if (leader) bulk_commit();
+    if (kTwoShot ? lane == 0 : leader) bulk_commit();
   }
 
-  if (leader) bulk_wait_done<0>();
+  if (kTwoShot ? lane == 0 : leader) bulk_wait_done<0>();
   __syncthreads();
   if (threadIdx.x == 0) io.ctrl[cta] = call + 1u;
 }

@@ -133,3 +133,25 @@ def test_default_team_width_per_shape():
     lib = N.cuda()
     assert lib.fp4ar_default_team_warps(4, 1) == 6 and lib.fp4ar_default_team_warps(8, 1) == 6
     assert lib.fp4ar_default_team_warps(2, 0) == 3 and lib.fp4ar_default_team_warps(2, 1) == 3 and lib.fp4ar_default_team_warps(4, 0) == 3
+
+
+@pytest.mark.parametrize("P", [1, 2, 4, 8])
+@pytest.mark.parametrize("inp,epi", [(N.IN_BF16, 0), (N.IN_BF16, 1), (N.IN_BF16, 2), (N.IN_NVFP4, 1), (N.IN_NVFP4, 3), (N.IN_NVFP4, 0)])
+def test_narrow_and_wide_shapes_at_their_limits(P, inp, epi):
+    """Up to two rows per CTA (and four, where the wide shape has three teams) run in the narrow build, the rest in the wide
+    one; calls of both alternate in one context, around every row count where the choice or the teams per CTA change."""
+    per = torch.cuda.get_device_properties(0).multi_processor_count // P        # CTAs of one emulated rank
+    rows = [1, per - 1, per, per + 1, 2 * per, 2 * per + 1, 3 * per + 1, 4 * per, 4 * per + 1, 7 * per + 5]
+    g = EmulatedGroup(P, max(rows))
+    g.set_timeout_ms(2000)
+    dev = torch.device("cuda", 0)
+    cells = [CellConfig(P, r, input=inp, epilogue=epi) for r in rows]
+    prepared = [(c, make_inputs(c, i, dev), Outputs(c, dev, P)) for i, c in enumerate(cells)]
+    for _ in range(2):
+        for c, data, outs in prepared:
+            outs.clear()
+            g.launch([args_for(c, data, outs, r, r) for r in range(P)])
+            torch.cuda.synchronize()
+            assert g.status(0).ok, g.status(0).describe()
+            assert sum(mismatches(c, data, outs, r) for r in range(P)) == 0, c
+    g.close()

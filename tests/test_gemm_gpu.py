@@ -41,7 +41,16 @@ def test_gemm_accumulators_and_quantised_rows(M, K, Nn, pair, monkeypatch):
 @pytest.mark.parametrize("P", [2, 4])
 def test_gemm_push_then_allreduce_on_emulated_ranks(P, pair, monkeypatch):
     monkeypatch.setenv("FP4AR_GEMM_PAIR", str(pair))
-    M, K = 256, 512
+    _push_then_allreduce(P, 256, 512)
+
+
+@pytest.mark.parametrize("P,M", [(2, 5), (2, 100), (4, 37), (8, 3), (8, 30)])
+def test_gemm_push_of_few_rows(P, M):
+    """Pushed rows finished by the narrow build of the AllReduce kernel (one or two rows per CTA)."""
+    _push_then_allreduce(P, M, 512)
+
+
+def _push_then_allreduce(P, M, K):
     g = EmulatedGroup(P, M)
     g.set_timeout_ms(500)
     xs, wts, gss, qs = [], [], [], []
