@@ -8,8 +8,8 @@
 //                 where the AllReduce kernel in "pushed input" mode finds them, and/or
 //               - into a local [M, N/2 + N/16] NVFP4 tensor.
 //
-// sm_100a structure: up to 256 rows the K loop of a tile is cut over a cluster (gemm_split_kernel below); above that
-// persistent CTAs (one per SM), K in blocks of 64, three shapes:
+// sm_100a structure: up to 384 rows one narrow tile per CTA (gemm_narrow_kernel below); above that persistent CTAs (one
+// per SM), K in blocks of 64, three shapes:
 //   pairs  (default for K >= 4096 or M >= 8192): the two CTAs of a cluster share one 256 x 256 tile with tcgen05
 //          cta_group::2: each loads its own 128 rows of A and half of the B block into a 6-stage ring, the even CTA
 //          issues the MMAs for both, each CTA's TMEM holds the accumulator of its own 128 rows;
@@ -50,7 +50,7 @@ constexpr int kBM = 128, kBK = 64;
 constexpr int kABytes = kBM * kBK * 2;            // 16 KB
 constexpr int kGemmThreads = 192;
 constexpr uint32_t kTmemCols = 512;
-constexpr int kMaxStages = 6, kSplitStages = 6;
+constexpr int kMaxStages = 6;
 
 // Tile width BN: 256 with a 4-stage ring, or 192 with a 5-stage ring.  With 148 persistent CTAs the tile count decides
 // how full the last wave is: M = 1024, N = 6144 gives 192 tiles of 128 x 256 (1.3 waves, 65 % busy) but 256 tiles of
@@ -90,8 +90,7 @@ struct GemmParams {
   StatusWords* status;
   unsigned long long timeout_ns;
   // split of the K loop across CTAs (see SegIter): partial accumulators and their flags, one slot per CTA
-  // few rows: CTAs of a cluster that share a tile's K loop, rows of the A box, ring stages (see gemm_split_kernel)
-  int split, a_rows, stages;
+  int a_rows, stages;    // few rows: rows of the A box, ring stages (see gemm_narrow_kernel)
   int stream_k;
   float* sk_partial;     // [grid][BN / 32][8][128] float4
   uint32_t* sk_flags;    // [grid][4]: 1 = the slot's quarter (32 rows) is written and not yet consumed
@@ -135,11 +134,6 @@ __device__ __forceinline__ uint32_t cluster_addr(const void* local, uint32_t ran
   uint32_t a;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(local)), "r"(rank));
   return a;
-}
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_smem) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_smem));
-  return v;
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
@@ -571,39 +565,44 @@ done:
   }
 }
 
-// Few rows (M <= 256): the K loop of a tile is cut over the CTAs of a cluster.
+// Few rows (M <= 384): one narrow tile per CTA, its whole K loop in one CTA.
 //
-// Such a call streams the weights once, and 24 - 48 CTAs with a whole K loop each do not draw the memory's bandwidth (about
-// 50 GB/s per SM whatever the ring's depth: M = 64, K = 8192 took 43 us for 100 MB).  Here S CTAs of a cluster take
-// K / S each of one 128 x BN tile, which fills the chip (N = 6144: 32 tiles of 192 columns x 4).  Every CTA then lays its
-// FP32 accumulator out in its own shared memory (over the idle ring), a cluster barrier makes them readable, and the CTAs
-// share the tile's rows: each adds the S partials of its rows in rank order through distributed shared memory, quantises
-// and stores.  No partial goes through global memory, no CTA waits for one that may not be resident (a cluster is
-// scheduled whole), and the order of the sum is fixed.  N = 6144, us, before -> now: M = 1: K = 1024 9.0 -> 5.5, K = 8192
-// 42.8 -> 19.6 (15.4 for the weights at the copy rate); M = 64: K = 2048 14.3 -> 8.8, K = 8192 43.3 -> 21.5; M = 128, K = 8192
-// 44.4 -> 23.4; M = 256, K = 8192 45.1 -> 32.9.
+// Such a call streams the weights once, and what bounds it is the chain of K blocks: a block of 64 takes a CTA about 300 ns
+// whatever the tile's width (wait, four MMAs into one accumulator, commit), so the time hardly depends on M or N.  Narrow
+// tiles of 128 x BN, BN 64 (up to 128 rows), 96 or 128 columns, put a CTA on most of the SMs (N = 6144: 96, 128 or 144 of
+// them) with a deep ring, a short set-up and a short epilogue that stores straight from registers.
+// The K loop is NOT cut over CTAs (a cluster of four that sums its partials takes half as long at K = 8192): the FP32
+// sums are then rounded elsewhere, about one value in 1e5 becomes another E2M1 value, and a step of the largest ones is
+// more than a normalised row may be off by.  Whole chains give the accumulators of the wide tiles bit for bit, so a row
+// does not change with the number of rows that share its call either.
+// N = 6144, us, 192- and 256-wide tiles -> now: M = 1: K = 1024 9.0 -> 7.5, K = 8192 45.3 -> 40.6; K = 2048: M = 16 14.5 -> 12.4,
+// M = 128 15.1 -> 12.8, M = 300 16.2 -> 14.0; K = 4096: M = 200 27.3 -> 23.2, M = 384 30.8 -> 26.9; M = 256, K = 8192 46.2 -> 45.2.
 // The A box holds only the valid rows, rounded up to eight: the MMA still takes 128 rows, and what it reads for the rest
-// is the start of the B block, whose products land in accumulator rows that nobody reads.
+// is the start of the B block or whatever follows it in shared memory, whose products land in accumulator rows that nobody
+// reads.
+constexpr int kNarrowStages = 16;
 template <int BN>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                  const __grid_constant__ GemmParams p) {
-  using S = GemmShape<BN, 1>;
+gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                   const __grid_constant__ GemmParams p) {
+  static_assert(BN == 64 || BN == 96 || BN == 128, "tile width");
+  constexpr int kBBytes = BN * kBK * 2;
+  constexpr uint32_t kCols = BN == 64 ? 64 : 128;       // TMEM columns, a power of two
+  constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  const int a_bytes = p.a_rows * kBK * 2, stage_bytes = a_bytes + S::kBBytes, stages = p.stages;
-  uint8_t* ring = smem;
-  uint64_t* full = reinterpret_cast<uint64_t*>(ring + stages * stage_bytes);   // [kSplitStages]
-  uint64_t* empty = full + kSplitStages;
-  uint64_t* acc_full = empty + kSplitStages;
+  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  const int a_bytes = p.a_rows * kBK * 2, stage_bytes = a_bytes + kBBytes, stages = p.stages;
+  // barriers beyond the 128 rows that the MMA reads from the last stage's A
+  uint64_t* full = reinterpret_cast<uint64_t*>(ring + (stages - 1) * stage_bytes + max(stage_bytes, kABytes));
+  uint64_t* empty = full + kNarrowStages;
+  uint64_t* acc_full = empty + kNarrowStages;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile uint32_t* abort_flag = tmem_holder + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int split = p.split, rank = (int)cluster_cta_rank(), tile = blockIdx.x / split;
-  const int n_tiles = p.N / BN, kblocks = p.K / kBK;
-  const int m0 = tile / n_tiles * kBM, n0 = tile % n_tiles * BN;
-  const int lo = kblocks * rank / split, count = kblocks * (rank + 1) / split - lo;
+  const int m_tiles = (p.M + kBM - 1) / kBM, kblocks = p.K / kBK;
+  // the tiles of one column range are neighbours: their weights cross HBM once
+  const int m0 = (int)blockIdx.x % m_tiles * kBM, n0 = (int)blockIdx.x / m_tiles * BN;
 
   if (threadIdx.x == 32) { prefetch_tensormap(&map_a); prefetch_tensormap(&map_b); }
   if (threadIdx.x == 0) {
@@ -612,7 +611,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     *abort_flag = 0u;
     mbar_init_fence();
   }
-  if (warp == 1) { tmem_alloc(tmem_holder, 256); tmem_relinquish(); }
+  if (warp == 1) { tmem_alloc(tmem_holder, kCols); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -622,12 +621,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   pdl_wait_prior_grids();
   pdl_release_dependents();
 
-  float4* const dump = reinterpret_cast<float4*>(ring);             // [BN / 4][a_rows]: lanes of a warp are consecutive rows
   if (warp == 0) {
     if (lane == 0) {
-      for (int it = 0; it < count; it++) {
-        const int st = it % stages;
-        if (!gemm_wait(empty + st, ((it / stages) & 1u) ^ 1u, gw, 1)) {
+      for (int it = 0, st = 0, round = 0; it < kblocks; it++) {
+        if (!gemm_wait(empty + st, (round & 1u) ^ 1u, gw, 1)) {
           // giving up: let the loads already issued land before the CTA (and its shared memory) goes away
           for (int back = 1; back <= stages && back <= it; back++) {
             uint32_t spins = 0;
@@ -636,105 +633,67 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           break;
         }
         mbar_arrive_expect(full + st, stage_bytes);
-        tma_load_2d(ring + st * stage_bytes, &map_a, (lo + it) * kBK, m0, full + st);
-        tma_load_2d(ring + st * stage_bytes + a_bytes, &map_b, (lo + it) * kBK, n0, full + st);
+        tma_load_2d(ring + st * stage_bytes, &map_a, it * kBK, m0, full + st);
+        tma_load_2d(ring + st * stage_bytes + a_bytes, &map_b, it * kBK, n0, full + st);
+        if (++st == stages) { st = 0; round++; }
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      bool good = true;
-      for (int it = 0; it < count && good; it++) {
-        const int st = it % stages;
-        good = gemm_wait(full + st, (it / stages) & 1u, gw, 3);
-        if (!good) break;
+      for (int it = 0, st = 0, round = 0; it < kblocks; it++) {
+        if (!gemm_wait(full + st, round & 1u, gw, 3)) break;
         tc_fence_after();
         const uint64_t da = umma_desc_k128(ring + st * stage_bytes), db = umma_desc_k128(ring + st * stage_bytes + a_bytes);
 #pragma unroll
         for (int k = 0; k < kBK / 16; k++)
-          umma_bf16(tmem_base, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), S::kIdesc, (it | k) != 0 ? 1u : 0u);
+          umma_bf16(tmem_base, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), kIdesc, (it | k) != 0 ? 1u : 0u);
         umma_commit(empty + st);
+        if (++st == stages) { st = 0; round++; }
       }
       umma_commit(acc_full);
     }
   } else {
-    const int q = warp & 3, row = q * 32 + lane;
+    const int q = warp & 3, row = m0 + q * 32 + lane;
     const bool good = __all_sync(0xffffffffu, gemm_wait(acc_full, 0u, gw, 4));
     tc_fence_after();
-    if (good && !*abort_flag && q * 32 < p.a_rows) {        // the ring is idle: every load was consumed by an MMA that has finished
+    if (good && !__any_sync(0xffffffffu, *abort_flag != 0u) && m0 + q * 32 < p.M) {
       const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16);
+      const int qrow_bytes = p.N / 2 + p.N / 16;
+      const size_t buf_off = p.nranks ? (size_t)(*p.call_counter & 1u) * p.buf_bytes : 0;
       float v[2][32];
       tmem_ld32_issue(tbase, v[0]);
 #pragma unroll
       for (int c = 0; c < BN / 32; c++) {
         tmem_ld_wait();
         if (c + 1 < BN / 32) tmem_ld32_issue(tbase + (c + 1) * 32, v[(c + 1) & 1]);
-        const float* vc = v[c & 1];
-        if (row < p.a_rows) {
+        float* vc = v[c & 1];
+        if (row < p.M) {
+          if (p.dbg_acc) {
+            float4* dst = reinterpret_cast<float4*>(p.dbg_acc + (size_t)row * p.N + n0 + c * 32);
 #pragma unroll
-          for (int i = 0; i < 8; i++) dump[(c * 8 + i) * p.a_rows + row] = make_float4(vc[4 * i], vc[4 * i + 1], vc[4 * i + 2], vc[4 * i + 3]);
+            for (int i = 0; i < 8; i++) dst[i] = make_float4(vc[4 * i], vc[4 * i + 1], vc[4 * i + 2], vc[4 * i + 3]);
+          }
+          uint4 qv;
+          const uint32_t sf2 = encode_pair_f32<true>(vc, [&](float b0, float b1, float& m0_, float& m1_) {
+            return pair_block_scales(b0, b1, p.inv_gs, m0_, m1_);
+          }, qv);
+          const size_t voff = (size_t)(n0 / 2 + 16 * c), soff = (size_t)(p.N / 2 + n0 / 16 + 2 * c);
+          auto put = [&](char* dst) {
+            *reinterpret_cast<uint4*>(dst + voff) = qv;
+            *reinterpret_cast<uint16_t*>(dst + soff) = (uint16_t)sf2;
+          };
+          if (p.local_q) put(p.local_q + (size_t)row * qrow_bytes);
+          if (p.nranks) {
+            if (p.two_shot) put(p.win[row % p.nranks] + buf_off + ((size_t)p.rank * p.capo + row / p.nranks) * kRecStride);
+            else for (int d = 0; d < p.nranks; d++) put(p.win[d] + buf_off + ((size_t)p.rank * p.cap + row) * kRecStride);
+          }
         }
       }
     }
   }
   tc_fence_before();
-  __syncwarp();
-  cluster_sync_all();                        // every CTA's partial is in its shared memory
-  tc_fence_after();
-  if (warp == 1) tmem_dealloc(tmem_base, 256);
-
-  // this CTA's rows of the tile: 16 columns of one row per thread and turn, neighbouring lanes on the two halves of a pair
-  const int valid = min(kBM, p.M - m0), per = (valid + split - 1) / split, r0 = rank * per, rows = max(0, min(per, valid - r0));
-  const int qrow_bytes = p.N / 2 + p.N / 16, items = rows * (BN / 16), half = lane & 1;
-  const size_t buf_off = p.nranks ? (size_t)(*p.call_counter & 1u) * p.buf_bytes : 0;
-  for (int base = warp * 32; base < items; base += kGemmThreads) {      // whole warps: the halves are exchanged below
-    const int item = min(base + lane, items - 2 + half) >> 1;
-    const int r = r0 + item % rows, c = item / rows, row = m0 + r;
-    float acc[16];
-    for (int s0 = 0; s0 < split; s0 += 4) {                             // four sources in flight
-      float4 f[4][4];
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-        if (s0 + u < split) {
-          const uint32_t a = cluster_addr(dump + (size_t)(c * 8 + half * 4) * p.a_rows + r, (uint32_t)(s0 + u));
-#pragma unroll
-          for (int i = 0; i < 4; i++) f[u][i] = ld_cluster_f4(a + (uint32_t)(i * p.a_rows * 16));
-        }
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-        if (s0 + u < split) {
-#pragma unroll
-          for (int i = 0; i < 4; i++) {
-            const float v[4] = {f[u][i].x, f[u][i].y, f[u][i].z, f[u][i].w};
-#pragma unroll
-            for (int e = 0; e < 4; e++) acc[4 * i + e] = s0 + u == 0 ? v[e] : __fadd_rn(acc[4 * i + e], v[e]);
-          }
-        }
-    }
-    const bool own = base + lane < items;
-    if (p.dbg_acc && own) {
-      float4* dst = reinterpret_cast<float4*>(p.dbg_acc + (size_t)row * p.N + n0 + c * 32 + half * 16);
-#pragma unroll
-      for (int i = 0; i < 4; i++) dst[i] = make_float4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
-    }
-    const float bm = absmax16(acc), other = __shfl_xor_sync(0xffffffffu, bm, 1);
-    float m0_, m1_;
-    const uint32_t sf2 = pair_block_scales(half ? other : bm, half ? bm : other, p.inv_gs, m0_, m1_);
-    const uint32_t w0 = quant_slot_f32<true>(acc, half ? m1_ : m0_), w1 = quant_slot_f32<true>(acc + 8, half ? m1_ : m0_);
-    const uint32_t w2 = __shfl_xor_sync(0xffffffffu, w0, 1), w3 = __shfl_xor_sync(0xffffffffu, w1, 1);
-    if (own && !half) {
-      const size_t voff = (size_t)(n0 / 2 + 16 * c), soff = (size_t)(p.N / 2 + n0 / 16 + 2 * c);
-      auto put = [&](char* dst) {
-        *reinterpret_cast<uint4*>(dst + voff) = make_uint4(w0, w1, w2, w3);
-        *reinterpret_cast<uint16_t*>(dst + soff) = (uint16_t)sf2;
-      };
-      if (p.local_q) put(p.local_q + (size_t)row * qrow_bytes);
-      if (p.nranks) {
-        if (p.two_shot) put(p.win[row % p.nranks] + buf_off + ((size_t)p.rank * p.capo + row / p.nranks) * kRecStride);
-        else for (int d = 0; d < p.nranks; d++) put(p.win[d] + buf_off + ((size_t)p.rank * p.cap + row) * kRecStride);
-      }
-    }
-  }
-  cluster_sync_all();                        // nobody leaves while its partial is still being read
+  __syncthreads();
+  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, kCols); }
 }
 
 // ---- host side ----
@@ -806,7 +765,7 @@ static bool stream_k_space(int slots, StreamKSpace* out) {
 using namespace fp4ar;
 
 // Which shape a call takes.  `units` = CTAs (or CTA pairs) that work, `tiles` = output tiles of that shape.
-struct GemmPlan { int pair, bn, stream_k, units, tiles, split; };
+struct GemmPlan { int pair, bn, stream_k, units, tiles, narrow; };
 static GemmPlan plan_gemm(int M, int N, int K, int sms, bool env) {
   // Tile width of single CTAs: the one whose tiles keep the persistent CTAs busier over all waves.  A 192-wide tile was
   // measured at about 0.87 of the per-cycle work of a 256-wide one (M = 4096: 321 vs 315 us at K = 8192 although its
@@ -814,13 +773,13 @@ static GemmPlan plan_gemm(int M, int N, int K, int sms, bool env) {
   // 192 too.  FP4AR_GEMM_TILE_N = 192 / 256 forces it (and single CTAs).
   int bn = 256;
   bool stream_k = false, pair = false;
-  // Few rows: clusters of `split` CTAs per tile (see gemm_split_kernel), where the tiles leave room for at least two each.
-  // An environment override of the shapes below switches it off.
-  if (!(env && (std::getenv("FP4AR_GEMM_TILE_N") || std::getenv("FP4AR_GEMM_STREAM_K") || std::getenv("FP4AR_GEMM_PAIR"))) && M <= 256) {
-    const int w = N % 192 == 0 ? 192 : 256, t = N / w * ((M + kBM - 1) / kBM);
-    int sp = 8;
-    while (sp > 1 && (t * sp > sms || K / kBK < sp)) sp /= 2;
-    if (sp > 1) return GemmPlan{0, w, 0, t, t, sp};
+  // Few rows: one narrow tile per CTA (see gemm_narrow_kernel), the widest of 128, 96 and 64 columns that gives two
+  // thirds of the SMs a tile and none of them two.  An environment override of the shapes below switches it off.
+  if (!(env && (std::getenv("FP4AR_GEMM_TILE_N") || std::getenv("FP4AR_GEMM_STREAM_K") || std::getenv("FP4AR_GEMM_PAIR"))) && M <= 384) {
+    for (int w : {128, 96, 64}) {
+      const int t = N / w * ((M + kBM - 1) / kBM);
+      if (N % w == 0 && (3 * t >= 2 * sms || w == 64) && t <= sms) return GemmPlan{0, w, 0, t, t, 1};
+    }
   }
   const char* force = env ? std::getenv("FP4AR_GEMM_TILE_N") : nullptr;
   const char* fsk = env ? std::getenv("FP4AR_GEMM_STREAM_K") : nullptr;
@@ -857,7 +816,7 @@ static GemmPlan plan_gemm(int M, int N, int K, int sms, bool env) {
     if (fsk) stream_k = std::atoi(fsk) != 0 && tiles > units && tiles % units != 0;
   }
   if (tiles < units) units = (int)tiles;
-  return GemmPlan{pair ? 1 : 0, bn, stream_k ? 1 : 0, units, (int)tiles, 1};
+  return GemmPlan{pair ? 1 : 0, bn, stream_k ? 1 : 0, units, (int)tiles, 0};
 }
 
 template <int BN, int G>
@@ -909,42 +868,34 @@ static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams 
 }
 
 template <int BN>
-static int launch_split(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int tiles, cudaStream_t stream) {
-  using S = GemmShape<BN, 1>;
-  const int stage = p.a_rows * kBK * 2 + S::kBBytes, dump = p.a_rows * BN * 4, tail = 256 + 1024;
-  // A ring as deep as the shared memory allows.  Short K ranges that manage with three stages in half of it (up to 64
-  // rows) take that: the next launch's CTAs then set up beside these (M = 16, K = 2048: 7.5 us against 7.8), while long
-  // ones want the bytes in flight (M = 64, K = 8192: 21.5 us with six stages, 23.8 with three; eight CTAs per tile, two per
-  // SM, 25.0).
-  constexpr int kHalf = 110 * 1024, kWhole = 220 * 1024;
-  p.stages = (kHalf - tail) / stage;
-  if (p.stages < 3 || p.K / kBK > 8 * p.split) p.stages = (kWhole - tail) / stage;
-  if (p.stages > kSplitStages) p.stages = kSplitStages;
-  const int smem = p.stages * stage + tail;
-  if (p.stages * stage < dump) return FP4AR_ERR_UNSUPPORTED;       // does not happen: three stages hold the dump of their rows
+static int launch_narrow(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int tiles, cudaStream_t stream) {
+  const int stage = (p.a_rows + BN) * kBK * 2, pad = stage < kABytes ? kABytes - stage : 0;
+  const int tail = 512 + 1024;                          // barriers, alignment slack
+  constexpr int kWhole = 224 * 1024;
+  p.stages = (kWhole - tail - pad) / stage;
+  if (p.stages > kNarrowStages) p.stages = kNarrowStages;
+  if (p.stages > p.K / kBK) p.stages = p.K / kBK;       // a short K loop leaves room for the next launch's CTAs
+  const int smem = p.stages * stage + pad + tail;
   static std::atomic<int> raised[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cuda_fail();
   if (!raised[dev].load(std::memory_order_acquire)) {
-    if (cudaFuncSetAttribute(gemm_split_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWhole) != cudaSuccess) return cuda_fail();
+    if (cudaFuncSetAttribute(gemm_narrow_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWhole) != cudaSuccess) return cuda_fail();
     raised[dev].store(1, std::memory_order_release);
   }
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.blockDim = dim3(kGemmThreads);
-  cfg.gridDim = dim3(tiles * p.split);
+  cfg.gridDim = dim3(tiles);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = p.split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
   const char* e = std::getenv("FP4AR_GEMM_PDL");
-  if (e && std::atoi(e) == 0) cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, gemm_split_kernel<BN>, ma, mb, p) != cudaSuccess) return cuda_fail();
+  cfg.numAttrs = e && std::atoi(e) == 0 ? 0 : 1;
+  if (cudaLaunchKernelEx(&cfg, gemm_narrow_kernel<BN>, ma, mb, p) != cudaSuccess) return cuda_fail();
   return cuda_check_launch();
 }
 
@@ -982,12 +933,12 @@ extern "C" int fp4ar_gemm_nvfp4(const fp4ar_push_view* push, int two_shot, const
     if (stream_k_space(device_sm_count(), &sp)) { p.stream_k = 1; p.sk_partial = sp.partial; p.sk_flags = sp.flags; }
   }
   CUtensorMap ma, mb;
-  if (pl.split > 1) {
-    p.split = pl.split;
+  if (pl.narrow) {
     p.a_rows = M < kBM ? (M + 7) / 8 * 8 : kBM;
     if (!make_map(&ma, x, M, K, p.a_rows) || !make_map(&mb, wt, N, K, bn)) return FP4AR_ERR_UNSUPPORTED;
-    return bn == 192 ? launch_split<192>(ma, mb, p, pl.tiles, (cudaStream_t)stream)
-                     : launch_split<256>(ma, mb, p, pl.tiles, (cudaStream_t)stream);
+    if (bn == 64) return launch_narrow<64>(ma, mb, p, pl.tiles, (cudaStream_t)stream);
+    return bn == 96 ? launch_narrow<96>(ma, mb, p, pl.tiles, (cudaStream_t)stream)
+                    : launch_narrow<128>(ma, mb, p, pl.tiles, (cudaStream_t)stream);
   }
   if (!make_map(&ma, x, M, K, kBM) || !make_map(&mb, wt, N, K, pair ? bn / 2 : bn)) return FP4AR_ERR_UNSUPPORTED;
   if (pair) return launch_gemm<256, 2>(ma, mb, p, (cudaStream_t)stream);

@@ -140,19 +140,22 @@ def test_gemm_reset_keeps_the_kernel_usable():
 
 
 @pytest.mark.parametrize("M,K,Nn", [(1, 1024, 6144), (8, 64 * 17, 6144), (9, 512, 6144), (64, 2048, 6144), (65, 512, 6144), (127, 8192, 6144),
-                                    (128, 256, 6144), (129, 576, 6144), (200, 128, 6144), (256, 4096, 6144), (33, 512, 256), (100, 64, 512),
-                                    (5, 192, 1024), (130, 320, 2048)])
-def test_gemm_of_few_rows_splits_k_over_a_cluster(M, K, Nn):
-    """Up to 256 rows the K loop is cut over a cluster (2, 4 or 8 CTAs, ragged ranges among them) and the partials are summed
-    through distributed shared memory; the FP32 sums of at most K products of N(0,1) / sqrt(K) terms stay within the bound
-    of the other shapes, the rows equal the host quantiser on the kernel's own sums, and a second call gives the same."""
+                                    (128, 256, 6144), (129, 576, 6144), (200, 128, 6144), (256, 4096, 6144), (257, 64, 6144), (384, 1024, 6144),
+                                    (33, 512, 256), (100, 64, 512), (5, 192, 1024), (130, 320, 2048)])
+def test_gemm_of_few_rows_equals_the_wide_tiles(M, K, Nn, monkeypatch):
+    """Up to 384 rows a CTA takes a narrow tile with its whole K loop: the same chain of MMAs per accumulator as in the
+    256-wide tiles, so sums and rows are the same bit for bit, and the rows equal the host quantiser on those sums."""
     x, wt = _xw(M, K, Nn, 7)
     gs = G.calibrate_gs(x, wt)
     q, acc = G.gemm_nvfp4(x, wt, gs, want_acc=True)
     q2 = G.gemm_nvfp4(x, wt, gs)
+    monkeypatch.setenv("FP4AR_GEMM_TILE_N", "256")
+    monkeypatch.setenv("FP4AR_GEMM_STREAM_K", "0")
+    wide, wide_acc = G.gemm_nvfp4(x, wt, gs, want_acc=True)
     torch.cuda.synchronize()
     assert G.gemm_status().code == 0
     ref = x.float() @ wt.float().t()
     assert (acc - ref).abs().max().item() <= 2e-3 * ref.abs().max().item() + 1e-4
     assert np.count_nonzero(q.cpu().numpy() != O.encode_static_f32(acc.cpu().numpy(), gs)) == 0
     assert torch.equal(q, q2)
+    assert torch.equal(acc, wide_acc) and torch.equal(q, wide)
