@@ -26,7 +26,7 @@ namespace fp4ar {
 // the area is transposed into "own pair" order through a bank-conflict-free swizzle.  A CTA is one team; several
 // CTAs share an SM (the kernels need no more than 12.5 KB of shared memory and 64-112 registers), so the loads of
 // one team overlap the arithmetic of the others.  Teams walk rows with a grid stride and take U rows per trip,
-// issuing every load of the trip before the first use.
+// issuing every load of the trip before the first use; where a row's work is long, the next row's loads are in flight meanwhile.
 // =============================================================================================
 constexpr int kTeamThreads = kPairs;          // 192
 constexpr int kTeamWarps = kTeamThreads / 32;  // 6
@@ -164,6 +164,12 @@ __host__ __device__ constexpr int decode_rows_per_trip(int ns, bool reenc) {
 // owner step 128 us at three teams with two rows per trip, 122 us at four with one.
 constexpr int kDecodeTeamsPerSm = 4;
 
+// The owner step works long enough on a row for the memory to idle meanwhile, so it loads its next row once the sum is in
+// the accumulators, for up to four sources, where the registers allow it (9000 rows, two sources 46.2 -> 41.0 us; 4096 rows,
+// four 28.0 -> 27.7; eight spill and lose, 41.0 -> 45.6).  The plain sum gains nothing by it (16384 rows, one source 45.7 either way;
+// 3001 rows, four 14.7 -> 15.7).
+__host__ __device__ constexpr bool decode_loads_ahead(int ns, bool reenc) { return reenc && ns <= 4; }
+
 template <int NS, bool REENC>
 __global__ void __launch_bounds__(kTeamThreads, kDecodeTeamsPerSm)
 decode_sum_kernel(SrcList src, long pitch, int rows, char* rec_out, char* out) {
@@ -175,20 +181,28 @@ decode_sum_kernel(SrcList src, long pitch, int rows, char* rec_out, char* out) {
   constexpr int U = decode_rows_per_trip(NS, REENC);
   pdl_wait_prior_grids();
   pdl_release_dependents();
+  constexpr bool kAhead = decode_loads_ahead(NS, REENC);
+  uint4 q[U][NS];
+  uint32_t sf[U][NS];
+  float rsv[U][NS];
+  auto load_row = [&](int u, int wanted) {
+    const int row = wanted < rows ? wanted : rows - 1;     // clamped: the extra loads are discarded
+#pragma unroll
+    for (int s = 0; s < NS; s++) {
+      const char* r = src.base[s] + (size_t)row * pitch;
+      q[u][s] = __ldcs(reinterpret_cast<const uint4*>(r + 16 * p));
+      sf[u][s] = __ldcs(reinterpret_cast<const unsigned short*>(r + kValueBytes + 2 * p));
+      rsv[u][s] = src.rs[s] ? __ldg(src.rs[s] + row) : src.gs[s];
+    }
+  };
+  if (kAhead) {
+#pragma unroll
+    for (int u = 0; u < U; u++) load_row(u, blockIdx.x * U + u);
+  }
   for (int row0 = blockIdx.x * U; row0 < rows; row0 += gridDim.x * U) {
-    uint4 q[U][NS];
-    uint32_t sf[U][NS];
-    float rsv[U][NS];
+    if (!kAhead) {
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      const int row = row0 + u < rows ? row0 + u : rows - 1;     // clamped: the extra loads are discarded
-#pragma unroll
-      for (int s = 0; s < NS; s++) {
-        const char* r = src.base[s] + (size_t)row * pitch;
-        q[u][s] = __ldcs(reinterpret_cast<const uint4*>(r + 16 * p));
-        sf[u][s] = __ldcs(reinterpret_cast<const unsigned short*>(r + kValueBytes + 2 * p));
-        rsv[u][s] = src.rs[s] ? __ldg(src.rs[s] + row) : src.gs[s];
-      }
+      for (int u = 0; u < U; u++) load_row(u, row0 + u);
     }
 #pragma unroll
     for (int u = 0; u < U; u++) {
@@ -198,6 +212,7 @@ decode_sum_kernel(SrcList src, long pitch, int rows, char* rec_out, char* out) {
       zero32(acc);
 #pragma unroll
       for (int s = 0; s < NS; s++) decode_acc_natural(acc, q[u][s], sf[u][s], rsv[u][s]);
+      if (kAhead && row + (int)gridDim.x * U < rows) load_row(u, row + gridDim.x * U);
       if (REENC) {
         float g6[kTeamWarps];
         const float bm0 = absmax16(acc), bm1 = absmax16(acc + 16);
@@ -233,33 +248,45 @@ decode_sum_kernel(SrcList src, long pitch, int rows, char* rec_out, char* out) {
 // add + Gemma RMSNorm:  z = x + res, res_out = bf16(z), y = (bf16(z) * rinv) * (wbias + w)
 // The sum of squares follows the fixed tree of the host model: per pair (t0 + t1) + (t2 + t3) over its four
 // chunk sums, a butterfly over the 32 pairs of a group (= one warp here), then the six groups in order.
+// Quantised outputs cost enough work per row that the memory idles during it: those shapes load a row ahead, with the
+// weights in shared memory to have the registers for it (16384 rows: NVFP4 out 118.5 -> 107.5 us, MXFP8 121.8 -> 116.6; 3000
+// rows, NVFP4 24.1 -> 21.7).  BF16 out runs at the copy rate as it is and loses by it (124.9 -> 139.7 us).
 // ---------------------------------------------------------------------------------------------
+__host__ __device__ constexpr bool norm_loads_ahead(int epi) { return epi >= 2; }
 template <int EPI>
 __global__ void __launch_bounds__(kTeamThreads, 3)
 add_rmsnorm_kernel(const char* __restrict__ x, const char* __restrict__ res_in, char* res_out,
                    const char* __restrict__ weight, float eps, float wbias, float qscale, char* out, char* outq,
                    int rows) {
   __shared__ __align__(128) uint8_t stage_all[kTeamWarps * kStageBytes];
+  __shared__ __align__(128) uint8_t weight_all[norm_loads_ahead(EPI) ? kTeamWarps * kStageBytes : 128];
   __shared__ float xchg[16];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, p = threadIdx.x;
   uint8_t* stage = stage_all + warp * kStageBytes;
   int phase = 0;
   pdl_wait_prior_grids();
   pdl_release_dependents();
+  constexpr bool kAhead = norm_loads_ahead(EPI);
+  uint4 rx[4], rr[4];
+  auto load_row = [&](int row) {
+    load_issue(x + (size_t)row * kRowB + warp * kStageBytes, lane, rx);
+    load_issue(res_in + (size_t)row * kRowB + warp * kStageBytes, lane, rr);
+  };
+  if (kAhead) load_row(blockIdx.x);                       // the grid has at most `rows` teams
   // this thread's 32 weights never change: fetched once
   uint4 wt[4];
+  uint8_t* wstage = kAhead ? weight_all + warp * kStageBytes : stage;
   {
     uint4 raw[4];
     load_issue(weight + warp * kStageBytes, lane, raw);
-    stage_in(stage, lane, raw, wt);
+    stage_in(wstage, lane, raw, wt);
   }
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-    uint4 rx[4], rr[4];
-    load_issue(x + (size_t)row * kRowB + warp * kStageBytes, lane, rx);
-    load_issue(res_in + (size_t)row * kRowB + warp * kStageBytes, lane, rr);
+    if (!kAhead) load_row(row);
     uint4 cx[4], cr[4];
     stage_in(stage, lane, rx, cx);
     stage_in(stage, lane, rr, cr);
+    if (kAhead && row + (int)gridDim.x < rows) load_row(row + gridDim.x);
     float acc[32];
     {
       const uint32_t* xw = reinterpret_cast<const uint32_t*>(cx);
@@ -276,6 +303,10 @@ add_rmsnorm_kernel(const char* __restrict__ x, const char* __restrict__ res_in, 
 #pragma unroll
     for (int g = 1; g < kTeamWarps; g++) ss = __fadd_rn(ss, g6[g]);
     const float rinv = norm_rinv(ss, eps);
+    if (kAhead) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) wt[k] = lds16(wstage + stage_off(lane, k));
+    }
     float y[32];
     norm_pair(zb, wt, rinv, wbias, y);
     uint4 yb[4];

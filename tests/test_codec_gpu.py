@@ -103,6 +103,28 @@ def test_add_rmsnorm_bit_exact(epi):
         assert np.count_nonzero(y.cpu().numpy() != want["outq"]) == 0
 
 
+@pytest.mark.parametrize("rows", [443, 444, 445, 592, 593, 1184, 1333])
+def test_rows_loaded_ahead_equal_rows_of_one_trip(rows):
+    """Calls of more rows than there are teams (444 of the norm, 592 of the codec on 148 SMs) load a row ahead: every row
+    equals the same row of calls that take one trip, at the edges of the trips, for the outputs that do so."""
+    x = D.partial(rows, 3).cuda()
+    res, w = D.residual(rows).cuda(), D.norm_weight().cuda()
+    for epi in (1, 2, 3):
+        whole_res = res.clone()
+        whole = codec.add_rmsnorm(x, whole_res, w, epilogue=epi, qscale=168.0, inplace_residual=True)[0]
+        for a in range(0, rows, 400):
+            part_res = res[a:a + 400].clone()
+            part = codec.add_rmsnorm(x[a:a + 400].clone(), part_res, w, epilogue=epi, qscale=168.0, inplace_residual=True)[0]
+            assert torch.equal(part, whole[a:a + 400]) and torch.equal(part_res, whole_res[a:a + 400])
+    rec = [codec.encode(D.partial(rows, 10 + s).cuda()) for s in range(5)]
+    for n in (2, 3, 4, 5):
+        q, rs = [r[0] for r in rec[:n]], [r[1] for r in rec[:n]]
+        got, out = codec.reduce_reencode(q, rs)
+        for a in range(0, rows, 400):
+            g, o = codec.reduce_reencode([t[a:a + 400].clone() for t in q], [t[a:a + 400].clone() for t in rs])
+            assert torch.equal(g, got[a:a + 400]) and torch.equal(o, out[a:a + 400])
+
+
 def test_fill_sentinel_pattern():
     buf = 3584 * 5 + 512   # five slots and a tail, two buffers
     buf = (buf + 4095) // 4096 * 4096
