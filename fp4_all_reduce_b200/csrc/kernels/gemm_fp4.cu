@@ -90,7 +90,7 @@ struct GemmParams {
   StatusWords* status;
   unsigned long long timeout_ns;
   // split of the K loop across CTAs (see SegIter): partial accumulators and their flags, one slot per CTA
-  int a_rows, stages;    // few rows: rows of the A box, ring stages (see gemm_narrow_kernel)
+  int a_rows, stages, atoms;    // few rows: rows of the A box, ring stages, K blocks per stage (see gemm_narrow_kernel)
   int stream_k;
   float* sk_partial;     // [grid][BN / 32][8][128] float4
   uint32_t* sk_flags;    // [grid][4]: 1 = the slot's quarter (32 rows) is written and not yet consumed
@@ -100,6 +100,12 @@ struct GemmParams {
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                ::"r"(smem_addr(smem_dst)), "l"(map), "r"(x), "r"(y), "r"(smem_addr(bar))
+               : "memory");
+}
+// `z` counts K blocks: a box of several lands as consecutive [rows][128 bytes] tiles
+__device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* map, int y, int z, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+               ::"r"(smem_addr(smem_dst)), "l"(map), "r"(0), "r"(y), "r"(z), "r"(smem_addr(bar))
                : "memory");
 }
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
@@ -567,16 +573,20 @@ done:
 
 // Few rows (M <= 384): one narrow tile per CTA, its whole K loop in one CTA.
 //
-// Such a call streams the weights once, and what bounds it is the chain of K blocks: a block of 64 takes a CTA about 300 ns
-// whatever the tile's width (wait, four MMAs into one accumulator, commit), so the time hardly depends on M or N.  Narrow
-// tiles of 128 x BN, BN 64 (up to 128 rows), 96 or 128 columns, put a CTA on most of the SMs (N = 6144: 96, 128 or 144 of
-// them) with a deep ring, a short set-up and a short epilogue that stores straight from registers.
+// Such a call streams the weights once, and what bounds it is the chain of ring stages: a stage of one K block of 64 takes a
+// CTA 300 - 400 ns whatever the tile's width and rows, one of two about 600, one of four about 950.  So a stage holds up to
+// four blocks, fetched by one copy per operand (the matrices are described as [K / 64][rows][64], a box of several blocks
+// lands as consecutive swizzled tiles), and the tiles are narrow: 128 x BN, BN 64 (up to 128 rows), 96 or 128 columns, put a
+// CTA on most of the SMs (N = 6144: 96, 128 or 144 of them), with a short set-up and a short epilogue that stores straight
+// from registers.  Where a stage holds one block the plain two-dimensional copies are the faster ones (M = 384, K = 4096:
+// 26.9 us against 29.9).
 // The K loop is NOT cut over CTAs (a cluster of four that sums its partials takes half as long at K = 8192): the FP32
 // sums are then rounded elsewhere, about one value in 1e5 becomes another E2M1 value, and a step of the largest ones is
 // more than a normalised row may be off by.  Whole chains give the accumulators of the wide tiles bit for bit, so a row
 // does not change with the number of rows that share its call either.
-// N = 6144, us, 192- and 256-wide tiles -> now: M = 1: K = 1024 9.0 -> 7.5, K = 8192 45.3 -> 40.6; K = 2048: M = 16 14.5 -> 12.4,
-// M = 128 15.1 -> 12.8, M = 300 16.2 -> 14.0; K = 4096: M = 200 27.3 -> 23.2, M = 384 30.8 -> 26.9; M = 256, K = 8192 46.2 -> 45.2.
+// N = 6144, us, 192- and 256-wide tiles -> one block per stage -> now: M = 1: K = 1024 14.3 -> 7.5 -> 6.0, K = 8192 45.3 -> 40.6 -> 30.3;
+// M = 16, K = 2048 14.5 -> 12.4 -> 9.7; K = 8192: M = 64 45.3 -> 40.9 -> 38.1, M = 128 45.6 -> 41.3 -> 38.2, M = 256 46.2 -> 45.2 -> 42.2;
+// M = 384, K = 4096 30.8 -> 26.9.
 // The A box holds only the valid rows, rounded up to eight: the MMA still takes 128 rows, and what it reads for the rest
 // is the start of the B block or whatever follows it in shared memory, whose products land in accumulator rows that nobody
 // reads.
@@ -591,16 +601,17 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  const int a_bytes = p.a_rows * kBK * 2, stage_bytes = a_bytes + kBBytes, stages = p.stages;
-  // barriers beyond the 128 rows that the MMA reads from the last stage's A
-  uint64_t* full = reinterpret_cast<uint64_t*>(ring + (stages - 1) * stage_bytes + max(stage_bytes, kABytes));
+  const int atoms = p.atoms, a_tile = p.a_rows * kBK * 2, a_bytes = atoms * a_tile, stage_bytes = a_bytes + atoms * kBBytes;
+  const int stages = p.stages;
+  // barriers beyond the 128 rows that the MMA reads from the last stage's last A tile
+  uint64_t* full = reinterpret_cast<uint64_t*>(ring + (stages - 1) * stage_bytes + max(stage_bytes, a_bytes - a_tile + kABytes));
   uint64_t* empty = full + kNarrowStages;
   uint64_t* acc_full = empty + kNarrowStages;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile uint32_t* abort_flag = tmem_holder + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m_tiles = (p.M + kBM - 1) / kBM, kblocks = p.K / kBK;
+  const int m_tiles = (p.M + kBM - 1) / kBM, kblocks = p.K / kBK, trips = (kblocks + atoms - 1) / atoms;
   // the tiles of one column range are neighbours: their weights cross HBM once
   const int m0 = (int)blockIdx.x % m_tiles * kBM, n0 = (int)blockIdx.x / m_tiles * BN;
 
@@ -623,7 +634,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
   if (warp == 0) {
     if (lane == 0) {
-      for (int it = 0, st = 0, round = 0; it < kblocks; it++) {
+      for (int it = 0, st = 0, round = 0; it < trips; it++) {
         if (!gemm_wait(empty + st, (round & 1u) ^ 1u, gw, 1)) {
           // giving up: let the loads already issued land before the CTA (and its shared memory) goes away
           for (int back = 1; back <= stages && back <= it; back++) {
@@ -633,20 +644,29 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           break;
         }
         mbar_arrive_expect(full + st, stage_bytes);
-        tma_load_2d(ring + st * stage_bytes, &map_a, it * kBK, m0, full + st);
-        tma_load_2d(ring + st * stage_bytes + a_bytes, &map_b, it * kBK, n0, full + st);
+        if (atoms > 1) {
+          tma_load_3d(ring + st * stage_bytes, &map_a, m0, it * atoms, full + st);
+          tma_load_3d(ring + st * stage_bytes + a_bytes, &map_b, n0, it * atoms, full + st);
+        } else {
+          tma_load_2d(ring + st * stage_bytes, &map_a, it * kBK, m0, full + st);
+          tma_load_2d(ring + st * stage_bytes + a_bytes, &map_b, it * kBK, n0, full + st);
+        }
         if (++st == stages) { st = 0; round++; }
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      for (int it = 0, st = 0, round = 0; it < kblocks; it++) {
+      for (int it = 0, st = 0, round = 0; it < trips; it++) {
         if (!gemm_wait(full + st, round & 1u, gw, 3)) break;
         tc_fence_after();
-        const uint64_t da = umma_desc_k128(ring + st * stage_bytes), db = umma_desc_k128(ring + st * stage_bytes + a_bytes);
+        uint64_t da = umma_desc_k128(ring + st * stage_bytes), db = umma_desc_k128(ring + st * stage_bytes + a_bytes);
+        const int n = min(atoms, kblocks - it * atoms);
+        for (int j = 0; j < n; j++) {
 #pragma unroll
-        for (int k = 0; k < kBK / 16; k++)
-          umma_bf16(tmem_base, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), kIdesc, (it | k) != 0 ? 1u : 0u);
+          for (int k = 0; k < kBK / 16; k++)
+            umma_bf16(tmem_base, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), kIdesc, (it | j | k) != 0 ? 1u : 0u);
+          da += (uint64_t)(a_tile >> 4); db += (uint64_t)(kBBytes >> 4);
+        }
         umma_commit(empty + st);
         if (++st == stages) { st = 0; round++; }
       }
@@ -719,6 +739,19 @@ static bool make_map(CUtensorMap* m, const void* base, int rows, int k, int box_
   cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// The same matrix as [K / 64][rows][64]: one box covers `atoms` K blocks.
+static bool make_map_3d(CUtensorMap* m, const void* base, int rows, int k, int box_rows, int atoms) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return false;
+  cuuint64_t dims[3] = {(cuuint64_t)kBK, (cuuint64_t)rows, (cuuint64_t)(k / kBK)};
+  cuuint64_t strides[2] = {(cuuint64_t)k * 2, (cuuint64_t)kBK * 2};
+  cuuint32_t box[3] = {(cuuint32_t)kBK, (cuuint32_t)box_rows, (cuuint32_t)atoms};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -869,12 +902,14 @@ static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams 
 
 template <int BN>
 static int launch_narrow(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int tiles, cudaStream_t stream) {
-  const int stage = (p.a_rows + BN) * kBK * 2, pad = stage < kABytes ? kABytes - stage : 0;
+  const int a_tile = p.a_rows * kBK * 2, stage = p.atoms * (a_tile + BN * kBK * 2);
+  const int last = (p.atoms - 1) * a_tile + kABytes, pad = stage < last ? last - stage : 0;     // what the MMA reads as A
   const int tail = 512 + 1024;                          // barriers, alignment slack
   constexpr int kWhole = 224 * 1024;
   p.stages = (kWhole - tail - pad) / stage;
   if (p.stages > kNarrowStages) p.stages = kNarrowStages;
-  if (p.stages > p.K / kBK) p.stages = p.K / kBK;       // a short K loop leaves room for the next launch's CTAs
+  const int trips = (p.K / kBK + p.atoms - 1) / p.atoms;
+  if (p.stages > trips) p.stages = trips;               // a short K loop leaves room for the next launch's CTAs
   const int smem = p.stages * stage + pad + tail;
   static std::atomic<int> raised[64];
   int dev = 0;
@@ -935,7 +970,12 @@ extern "C" int fp4ar_gemm_nvfp4(const fp4ar_push_view* push, int two_shot, const
   CUtensorMap ma, mb;
   if (pl.narrow) {
     p.a_rows = M < kBM ? (M + 7) / 8 * 8 : kBM;
-    if (!make_map(&ma, x, M, K, p.a_rows) || !make_map(&mb, wt, N, K, bn)) return FP4AR_ERR_UNSUPPORTED;
+    // K blocks per stage: as many, up to four, as leave the ring at least four stages deep
+    p.atoms = 4;
+    while (p.atoms > 1 && (p.atoms > K / kBK || p.atoms * (p.a_rows + bn) * kBK * 2 > 56 * 1024)) p.atoms /= 2;
+    const bool maps = p.atoms > 1 ? make_map_3d(&ma, x, M, K, p.a_rows, p.atoms) && make_map_3d(&mb, wt, N, K, bn, p.atoms)
+                                  : make_map(&ma, x, M, K, p.a_rows) && make_map(&mb, wt, N, K, bn);
+    if (!maps) return FP4AR_ERR_UNSUPPORTED;
     if (bn == 64) return launch_narrow<64>(ma, mb, p, pl.tiles, (cudaStream_t)stream);
     return bn == 96 ? launch_narrow<96>(ma, mb, p, pl.tiles, (cudaStream_t)stream)
                     : launch_narrow<128>(ma, mb, p, pl.tiles, (cudaStream_t)stream);

@@ -140,7 +140,7 @@ def test_gemm_reset_keeps_the_kernel_usable():
 
 
 @pytest.mark.parametrize("M,K,Nn", [(1, 1024, 6144), (8, 64 * 17, 6144), (9, 512, 6144), (64, 2048, 6144), (65, 512, 6144), (127, 8192, 6144),
-                                    (128, 256, 6144), (129, 576, 6144), (200, 128, 6144), (256, 4096, 6144), (257, 64, 6144), (384, 1024, 6144),
+                                    (24, 64, 6144), (40, 64 * 5, 6144), (56, 64 * 6, 6144), (120, 64 * 3, 6144), (128, 256, 6144), (129, 576, 6144), (200, 128, 6144), (256, 4096, 6144), (257, 64, 6144), (384, 1024, 6144),
                                     (33, 512, 256), (100, 64, 512), (5, 192, 1024), (130, 320, 2048)])
 def test_gemm_of_few_rows_equals_the_wide_tiles(M, K, Nn, monkeypatch):
     """Up to 384 rows a CTA takes a narrow tile with its whole K loop: the same chain of MMAs per accumulator as in the
