@@ -578,15 +578,14 @@ done:
 // four blocks, fetched by one copy per operand (the matrices are described as [K / 64][rows][64], a box of several blocks
 // lands as consecutive swizzled tiles), and the tiles are narrow: 128 x BN, BN 64 (up to 128 rows), 96 or 128 columns, put a
 // CTA on most of the SMs (N = 6144: 96, 128 or 144 of them), with a short set-up and a short epilogue that stores straight
-// from registers.  Where a stage holds one block the plain two-dimensional copies are the faster ones (M = 384, K = 4096:
-// 26.9 us against 29.9).
+// from registers.
 // The K loop is NOT cut over CTAs (a cluster of four that sums its partials takes half as long at K = 8192): the FP32
 // sums are then rounded elsewhere, about one value in 1e5 becomes another E2M1 value, and a step of the largest ones is
 // more than a normalised row may be off by.  Whole chains give the accumulators of the wide tiles bit for bit, so a row
 // does not change with the number of rows that share its call either.
 // N = 6144, us, 192- and 256-wide tiles -> one block per stage -> now: M = 1: K = 1024 14.3 -> 7.5 -> 6.0, K = 8192 45.3 -> 40.6 -> 30.3;
-// M = 16, K = 2048 14.5 -> 12.4 -> 9.7; K = 8192: M = 64 45.3 -> 40.9 -> 38.1, M = 128 45.6 -> 41.3 -> 38.2, M = 256 46.2 -> 45.2 -> 42.2;
-// M = 384, K = 4096 30.8 -> 26.9.
+// M = 16, K = 2048 14.5 -> 12.4 -> 9.7; K = 8192: M = 64 45.4 -> 40.8 -> 30.7, M = 384 56.1 -> 51.2 -> 49.5;
+// K = 4096: M = 200 27.2 -> 23.3 -> 22.7, M = 384 31.0 -> 26.9 -> 26.2; K = 2048: M = 128 15.0 -> 12.7 -> 10.8, M = 300 16.3 -> 14.0 -> 13.6.
 // The A box holds only the valid rows, rounded up to eight: the MMA still takes 128 rows, and what it reads for the rest
 // is the start of the B block or whatever follows it in shared memory, whose products land in accumulator rows that nobody
 // reads.
@@ -970,9 +969,9 @@ extern "C" int fp4ar_gemm_nvfp4(const fp4ar_push_view* push, int two_shot, const
   CUtensorMap ma, mb;
   if (pl.narrow) {
     p.a_rows = M < kBM ? (M + 7) / 8 * 8 : kBM;
-    // K blocks per stage: as many, up to four, as leave the ring at least four stages deep
+    // K blocks per stage: as many, up to four, as leave the ring two stages (M = 64, K = 8192: 30.7 us, with four shorter stages 38.1)
     p.atoms = 4;
-    while (p.atoms > 1 && (p.atoms > K / kBK || p.atoms * (p.a_rows + bn) * kBK * 2 > 56 * 1024)) p.atoms /= 2;
+    while (p.atoms > 1 && (p.atoms > K / kBK || p.atoms * (p.a_rows + bn) * kBK * 2 > 100 * 1024)) p.atoms /= 2;
     const bool maps = p.atoms > 1 ? make_map_3d(&ma, x, M, K, p.a_rows, p.atoms) && make_map_3d(&mb, wt, N, K, bn, p.atoms)
                                   : make_map(&ma, x, M, K, p.a_rows) && make_map(&mb, wt, N, K, bn);
     if (!maps) return FP4AR_ERR_UNSUPPORTED;
