@@ -72,6 +72,10 @@ inline bool layout_ok(const Tensor& t, at::ScalarType dtype, int64_t cols) {
 inline void require(const Tensor& t, at::ScalarType dtype, int64_t cols, const char* name) {
   if (!layout_ok(t, dtype, cols) || !t.is_cuda()) bad_layout(t, dtype, cols, name);
 }
+// The kernels trust their pointers: every tensor of a call lives on the device that it is launched on.
+inline void require_on(const Tensor& t, c10::Device dev, const char* name) {
+  TORCH_CHECK_VALUE(t.device() == dev, name, " is on ", t.device(), ", the call runs on ", dev);
+}
 
 inline Tensor new_empty(at::IntArrayRef size, at::ScalarType dtype, c10::Device dev) {
   return Tensor(at::detail::empty_cuda(size, dtype, dev, std::nullopt));
@@ -126,6 +130,7 @@ Sources sources(const std::vector<Tensor>& q, const std::vector<Tensor>& row_sca
   if (s.pitch < 0) bad_layout(q[0], at::kByte, kQRow, "source");
   for (const Tensor& t : q) {
     require(t, at::kByte, s.pitch, "source");
+    require_on(t, q[0].device(), "source");
     TORCH_CHECK_VALUE(t.sizes() == q[0].sizes(), "sources must have one shape");
   }
   TORCH_CHECK_VALUE(s.pitch == kQRow || s.pitch == kRec, "source rows must be 3456 B (NVFP4 rows) or 3584 B (receive records)");
@@ -136,6 +141,8 @@ Sources sources(const std::vector<Tensor>& q, const std::vector<Tensor>& row_sca
     s.rs[i] = nullptr;
     if (!row_scales.empty() && row_scales[i].defined()) {
       require(row_scales[i], at::kFloat, -1, "row_scales");
+      require_on(row_scales[i], q[0].device(), "row_scales");
+      TORCH_CHECK_VALUE(row_scales[i].numel() >= s.rows, "row_scales must have ", s.rows, " elements, got ", row_scales[i].numel());
       s.rs[i] = (const float*)row_scales[i].data_ptr();
     } else {
       TORCH_CHECK_VALUE(have_gs, "a source without row scales needs a static scale");
@@ -167,22 +174,30 @@ std::tuple<Tensor, Tensor> op_reduce_reencode(const std::vector<Tensor>& q, cons
   return {std::move(rec), std::move(out)};
 }
 
-// `out` undefined: allocated.  `inplace`: the updated residual replaces `residual`.
+// `out` undefined: allocated; given: any contiguous memory of the device that holds the rows.  `inplace`: the updated
+// residual replaces `residual`.
 std::tuple<Tensor, Tensor> op_norm(const Tensor& x, const Tensor& residual, const Tensor& weight, double eps, double weight_bias,
                                    int64_t epilogue, double qscale, bool inplace, Tensor out) {
   require(x, at::kBFloat16, kHidden, "x");
   require(residual, at::kBFloat16, kHidden, "residual");
-  TORCH_CHECK_VALUE(weight.scalar_type() == at::kBFloat16 && weight.numel() == kHidden && weight.is_cuda(),
-                    "weight must be a CUDA BF16 tensor of 6144 elements");
+  TORCH_CHECK_VALUE(weight.scalar_type() == at::kBFloat16 && weight.numel() == kHidden && weight.is_cuda() && weight.is_contiguous(),
+                    "weight must be a contiguous CUDA BF16 tensor of 6144 elements");
   const int64_t rows = x.size(0);
   TORCH_CHECK_VALUE(residual.size(0) >= rows, "residual must have ", rows, " rows, got ", residual.size(0));
   TORCH_CHECK_VALUE(epilogue >= FP4AR_EPI_NORM_BF16 && epilogue <= FP4AR_EPI_NORM_MXFP8, "epilogue must be 1 (BF16), 2 (NVFP4) or 3 (MXFP8)");
   const c10::Device dev = x.device();
-  const c10::cuda::CUDAGuard guard(dev);
-  Tensor res_out = inplace ? residual : new_empty(residual.sizes(), at::kBFloat16, residual.device());
+  require_on(residual, dev, "residual");
+  require_on(weight, dev, "weight");
   const bool bf16 = epilogue == FP4AR_EPI_NORM_BF16;
-  if (!out.defined())
-    out = bf16 ? new_empty(x.sizes(), at::kBFloat16, dev) : new_empty({rows, epilogue == FP4AR_EPI_NORM_NVFP4 ? kQRow : kMxRow}, at::kByte, dev);
+  const int64_t cols = bf16 ? kHidden : epilogue == FP4AR_EPI_NORM_NVFP4 ? kQRow : kMxRow;
+  if (out.defined()) {
+    const int64_t bytes = rows * cols * (bf16 ? 2 : 1);
+    TORCH_CHECK_VALUE(out.device() == dev && out.is_contiguous() && (int64_t)out.nbytes() >= bytes,
+                      "out must be contiguous, on ", dev, " and hold ", bytes, " bytes");
+  }
+  const c10::cuda::CUDAGuard guard(dev);
+  Tensor res_out = inplace ? residual : new_empty(residual.sizes(), at::kBFloat16, dev);
+  if (!out.defined()) out = new_empty({rows, cols}, bf16 ? at::kBFloat16 : at::kByte, dev);
   void* op = out.mutable_data_ptr();
   ok(api.add_rmsnorm(x.data_ptr(), residual.data_ptr(), res_out.mutable_data_ptr(), weight.data_ptr(), (float)eps, (float)weight_bias,
                      (int)epilogue, (float)qscale, bf16 ? op : nullptr, bf16 ? nullptr : op, (int)rows, stream_of(dev)),
@@ -198,6 +213,7 @@ std::tuple<Tensor, Tensor> op_gemm(const Tensor& x, const Tensor& wt, double gs,
   const int64_t M = x.size(0), K = x.size(1), Nn = wt.size(0);
   TORCH_CHECK_VALUE(K % 64 == 0 && Nn % 256 == 0, "K must be a multiple of 64 and N a multiple of 256");
   const c10::Device dev = x.device();
+  require_on(wt, dev, "wt");
   const c10::cuda::CUDAGuard guard(dev);
   const int64_t qb = Nn / 2 + Nn / 16;
   if (!q.defined()) {

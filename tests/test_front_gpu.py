@@ -1,0 +1,90 @@
+"""Argument checks of the native front end: an argument that the kernels could not trust raises by name before any launch."""
+import pytest
+import torch
+
+from fp4_all_reduce_b200 import _native as N
+from fp4_all_reduce_b200.ops import allreduce as A  # noqa: F401  (registers torch.ops.fp4ar)
+from fp4_all_reduce_b200.ops import codec
+from fp4_all_reduce_b200.ops import gemm as G
+
+pytestmark = pytest.mark.gpu
+
+ROWS = 8
+
+
+def _bf16(rows=ROWS, cols=N.HIDDEN, device="cuda"):
+    return torch.zeros(rows, cols, dtype=torch.bfloat16, device=device)
+
+
+def test_norm_takes_only_memory_that_holds_its_rows():
+    x, res, w = _bf16(), _bf16(), _bf16(1).view(-1)
+    bad_out = {
+        1: [_bf16(ROWS - 1), _bf16(device="cpu"), _bf16(ROWS, 2 * N.HIDDEN)[:, ::2]],
+        2: [torch.zeros(ROWS, N.QROW_BYTES - 16, dtype=torch.uint8, device="cuda"), torch.zeros(ROWS, N.QROW_BYTES, dtype=torch.uint8)],
+        3: [torch.zeros(ROWS, N.QROW_BYTES, dtype=torch.uint8, device="cuda")],
+    }
+    for epi, outs in bad_out.items():
+        for out in outs:
+            with pytest.raises(ValueError, match="out must be"):
+                codec.add_rmsnorm(x, res, w, epilogue=epi, out=out)
+    for bad_w in (_bf16(2).view(-1)[::2], torch.zeros(1, dtype=torch.bfloat16, device="cuda").expand(N.HIDDEN), w.cpu(), w[:100]):
+        with pytest.raises(ValueError, match="weight must be"):
+            codec.add_rmsnorm(x, res, bad_w)
+    with pytest.raises(ValueError, match="residual must have"):
+        codec.add_rmsnorm(x, res[:ROWS - 1], w)
+    with pytest.raises(ValueError, match="residual"):
+        codec.add_rmsnorm(x, res.cpu(), w)
+    with pytest.raises(ValueError, match="epilogue"):
+        codec.add_rmsnorm(x, res, w, epilogue=4)
+    with pytest.raises(ValueError, match="residual must have"):
+        torch.ops.fp4ar.add_rms_norm(x, res[:1], w, 1e-6, 1.0)
+    out = _bf16(ROWS + 3)                                  # room for more rows than the call has: the rest is left alone
+    out.fill_(7)
+    y, _ = codec.add_rmsnorm(x + 1, res, w, out=out)
+    assert y is out and torch.all(out[ROWS:] == 7) and torch.all(out[:ROWS] != 7)
+
+
+def test_sources_of_a_sum_bring_enough_row_scales_on_the_same_device():
+    q, rs = codec.encode(_bf16() + 1)
+    for fn in (codec.decode_sum, codec.reduce_reencode, lambda a, b: torch.ops.fp4ar.decode_sum(a, b)):
+        with pytest.raises(ValueError, match="row_scales must have 8 elements"):
+            fn([q, q], [rs, rs[:ROWS - 1]])
+        with pytest.raises((ValueError, NotImplementedError, RuntimeError)):
+            fn([q, q], [rs, rs.cpu()])
+        with pytest.raises((ValueError, NotImplementedError, RuntimeError)):
+            fn([q, q.cpu()], [rs, rs])
+        with pytest.raises(ValueError, match="one shape"):
+            fn([q, q[:2]], [rs, rs])
+        with pytest.raises(ValueError, match="3456"):
+            fn([q[:, :3072].contiguous()], [rs])
+    with pytest.raises(ValueError, match="static scale"):
+        codec.decode_sum([q])
+    with pytest.raises(ValueError, match="1..8"):
+        codec.decode_sum([])
+
+
+@pytest.mark.multigpu
+def test_tensors_of_another_device_are_refused():
+    x, res, w = _bf16(), _bf16(), _bf16(1).view(-1)
+    there = "cuda:1"
+    for args in ((x, res.to(there), w), (x, res, w.to(there))):
+        with pytest.raises(ValueError, match="is on cuda:1"):
+            codec.add_rmsnorm(*args)
+    q, rs = codec.encode(x)
+    with pytest.raises(ValueError, match="is on cuda:1"):
+        codec.decode_sum([q, q.to(there)], [rs, rs])
+    with pytest.raises(ValueError, match="is on cuda:1"):
+        codec.decode_sum([q, q], [rs, rs.to(there)])
+    with pytest.raises(ValueError, match="is on cuda:1"):
+        G.gemm_nvfp4(_bf16(ROWS, 64), _bf16(N.HIDDEN, 64, there), 1.0)
+
+
+def test_gemm_arguments():
+    x, wt = _bf16(ROWS, 128), _bf16(N.HIDDEN, 128)
+    for bad in ((x[:, :64], wt), (x, wt[:, :64]), (x, wt.cpu()), (x.float(), wt), (x, _bf16(100, 128))):
+        with pytest.raises(ValueError):
+            G.gemm_nvfp4(*bad, 1.0)
+    for out in (torch.zeros(ROWS - 1, N.QROW_BYTES, dtype=torch.uint8, device="cuda"), torch.zeros(ROWS, N.QROW_BYTES, dtype=torch.uint8),
+                torch.zeros(ROWS, N.QROW_BYTES, dtype=torch.int8, device="cuda")):
+        with pytest.raises(ValueError, match="out must be"):
+            G.gemm_nvfp4(x, wt, 1.0, out=out)
