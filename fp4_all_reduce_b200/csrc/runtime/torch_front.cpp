@@ -146,7 +146,6 @@ Sources sources(const std::vector<Tensor>& q, const std::vector<Tensor>& row_sca
       s.rs[i] = (const float*)row_scales[i].data_ptr();
     } else {
       TORCH_CHECK_VALUE(have_gs, "a source without row scales needs a static scale");
-      TORCH_CHECK_INDEX(i < (int)gs.size(), "list index out of range");
       s.gs[i] = (float)gs[i];
     }
   }
@@ -289,7 +288,8 @@ void each(PyObject* seq, F&& f) {
   const Py_ssize_t n = PySequence_Fast_GET_SIZE(fast.get());
   for (Py_ssize_t i = 0; i < n; i++) f(PySequence_Fast_GET_ITEM(fast.get(), i));
 }
-// (qrows, row_scales or None, gs or None)
+// (qrows, row_scales or None, gs or None).  Only the static scales of sources without row scales are looked at: the entries
+// of the others may be anything, None among them.
 struct SourceArgs {
   std::vector<Tensor> q, rs;
   std::vector<double> gs;
@@ -301,7 +301,14 @@ struct SourceArgs {
       rs.reserve(FP4AR_MAX_RANKS);
       each(a[1], [&](PyObject* o) { if (o == Py_None) rs.emplace_back(); else rs.push_back(tensor_arg(o, "row_scales")); });
     }
-    if (have_gs) each(a[2], [&](PyObject* o) { gs.push_back(double_arg(o)); });
+    if (!have_gs) return;
+    gs.resize(q.size());
+    for (size_t i = 0; i < q.size(); i++) {
+      if (a[1] != Py_None && (i >= rs.size() || rs[i].defined())) continue;
+      THPObjectPtr key(PyLong_FromSize_t(i)), item(key ? PyObject_GetItem(a[2], key.get()) : nullptr);
+      if (!item) throw python_error();
+      gs[i] = double_arg(item.get());
+    }
   }
 };
 PyObject* py_decode_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {

@@ -133,3 +133,25 @@ def test_zero_row_call_and_poisoned_code_have_names():
     assert N.ERROR_NAMES[4] == "context poisoned"
     with pytest.raises(N.ContextPoisoned):
         N.check(4, "fp4ar_launch")
+
+
+@pytest.fixture(scope="module")
+def front(cuda_lib):
+    """The native front end on host tensors: what it does before its device checks needs no GPU."""
+    try:
+        return N.front()
+    except (RuntimeError, OSError, ImportError) as e:
+        pytest.skip(str(e))
+
+
+def test_static_scales_are_read_only_for_sources_without_row_scales(front):
+    """A list of scales may hold anything in the places of sources that bring row scales, as in `gs[i]` of plain Python."""
+    q, rs = torch.zeros(3, 3456, dtype=torch.uint8), torch.ones(3)
+    for gs in ([None, 0.5], ("unused", 0.5), {1: 0.5}, torch.tensor([float("nan"), 0.5])):
+        for fn in (front.decode_sum, front.reduce_reencode):
+            with pytest.raises(ValueError, match="CUDA"):          # the first complaint is that these are host tensors
+                fn([q, q], [rs, None], gs)
+    with pytest.raises(IndexError):
+        front.decode_sum([q, q], None, [0.5])
+    with pytest.raises(TypeError):
+        front.decode_sum([q, q], [None, rs], [None, 0.5])
