@@ -250,6 +250,11 @@ int64_t int_arg(PyObject* o) {
   if (v == -1 && PyErr_Occurred()) throw python_error();
   return v;
 }
+bool bool_arg(PyObject* o) {
+  const int v = PyObject_IsTrue(o);
+  if (v < 0) throw python_error();
+  return v != 0;
+}
 void arity(Py_ssize_t got, Py_ssize_t want) {
   if (got != want) throw torch::TypeError("expected " + std::to_string(want) + " arguments, got " + std::to_string(got));
 }
@@ -333,9 +338,9 @@ PyObject* py_add_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const Tensor &x = tensor_arg(a[0], "x"), &res = tensor_arg(a[1], "residual"), &w = tensor_arg(a[2], "weight");
   const double eps = double_arg(a[3]), wb = double_arg(a[4]), qs = double_arg(a[6]);
   const int64_t epi = int_arg(a[5]);
-  const int inplace = PyObject_IsTrue(a[7]);
+  const bool inplace = bool_arg(a[7]);
   Tensor out = a[8] == Py_None ? Tensor() : tensor_arg(a[8], "out");
-  auto r = [&] { NoGil g; return op_norm(x, res, w, eps, wb, epi, qs, inplace != 0, std::move(out)); }();
+  auto r = [&] { NoGil g; return op_norm(x, res, w, eps, wb, epi, qs, inplace, std::move(out)); }();
   return wrap2(std::move(std::get<0>(r)), std::move(std::get<1>(r)));
   END_HANDLE_TH_ERRORS
 }
@@ -345,7 +350,7 @@ PyObject* py_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   arity(n, 5);
   const Tensor &x = tensor_arg(a[0], "x"), &wt = tensor_arg(a[1], "wt");
   const double gs = double_arg(a[2]);
-  const bool acc = PyObject_IsTrue(a[3]) != 0;
+  const bool acc = bool_arg(a[3]);
   Tensor out = a[4] == Py_None ? Tensor() : tensor_arg(a[4], "out");
   auto r = [&] { NoGil g; return op_gemm(x, wt, gs, acc, std::move(out)); }();
   if (!acc) return THPVariable_Wrap(std::move(std::get<0>(r)));
@@ -377,10 +382,16 @@ inline bool get_int(PyObject* o, int& v) {
   return !over && l == (long)v;
 }
 inline bool get_float(PyObject* o, float& v) {
-  if (PyFloat_Check(o)) v = (float)PyFloat_AS_DOUBLE(o);
-  else if (PyLong_CheckExact(o)) v = (float)PyLong_AsDouble(o);
-  else return false;
-  return true;
+  if (PyFloat_Check(o)) {
+    v = (float)PyFloat_AS_DOUBLE(o);
+    return true;
+  }
+  if (!PyLong_CheckExact(o)) return false;
+  const double d = PyLong_AsDouble(o);
+  v = (float)d;
+  if (d != -1.0 || !PyErr_Occurred()) return true;
+  PyErr_Clear();                 // beyond a double: the Python wrapper raises it
+  return false;
 }
 
 // The input (BF16 rows or NVFP4 rows with one positive scale per rank) and the options every call has.

@@ -6,6 +6,7 @@ from fp4_all_reduce_b200 import _native as N
 from fp4_all_reduce_b200.ops import allreduce as A  # noqa: F401  (registers torch.ops.fp4ar)
 from fp4_all_reduce_b200.ops import codec
 from fp4_all_reduce_b200.ops import gemm as G
+from fp4_all_reduce_b200.parallel.context import SoloRankContext
 
 pytestmark = pytest.mark.gpu
 
@@ -88,3 +89,10 @@ def test_gemm_arguments():
                 torch.zeros(ROWS, N.QROW_BYTES, dtype=torch.int8, device="cuda")):
         with pytest.raises(ValueError, match="out must be"):
             G.gemm_nvfp4(x, wt, 1.0, out=out)
+
+
+def test_a_number_beyond_a_double_is_an_overflow():
+    ctx = SoloRankContext(2, ROWS)
+    with pytest.raises(OverflowError):
+        ctx.all_reduce_add_rms_norm(_bf16(), _bf16(), _bf16(1).view(-1), eps=10**400, mode=N.MODE_COMPUTE)
+    ctx.close()

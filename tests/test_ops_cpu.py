@@ -155,3 +155,11 @@ def test_static_scales_are_read_only_for_sources_without_row_scales(front):
         front.decode_sum([q, q], None, [0.5])
     with pytest.raises(TypeError):
         front.decode_sum([q, q], [None, rs], [None, 0.5])
+
+
+def test_a_flag_without_a_truth_value_raises_its_own_error(front):
+    x, w = torch.zeros(3, 6144, dtype=torch.bfloat16), torch.zeros(6144, dtype=torch.bfloat16)
+    with pytest.raises(RuntimeError, match="ambiguous"):
+        front.add_rmsnorm(x, x, w, 1e-6, 1.0, 1, 1.0, torch.ones(2), None)
+    with pytest.raises(RuntimeError, match="ambiguous"):
+        front.gemm(x, x, 1.0, torch.ones(2), None)
