@@ -26,8 +26,14 @@ int fp4ar_gemm_nvfp4(const fp4ar_push_view* push, int two_shot, const void* x, c
 /* Status block of the GEMM kernels on the current device (code != 0: a bounded wait gave up). */
 int fp4ar_gemm_status(fp4ar_status_words* out);
 /* After a GEMM whose status is not 0: waits for the device, then clears the status block and the hand-off flags of the
- * partial tiles that such a launch may have left set (a later launch would wait on them until its limit). */
+ * partial tiles that such a launch may have left set (a later launch would wait on them until its limit).  Workspaces
+ * that no graph owns are freed. */
 int fp4ar_gemm_reset(void);
+/* The workspace of partial tiles that a launch with a cut K loop takes on `stream` (allocated if need be; while the stream
+ * is being captured, the one its graph will own).  Launches that may run at the same time have different ones: launches of
+ * different streams, of a graph and a stream, of different graphs.  Instances of one captured graph share theirs, so only
+ * one of them may run at a time (and an instance updated from another graph needs both graphs kept).  NULL: none could be had, a launch then runs whole tiles. */
+const void* fp4ar_gemm_workspace(fp4ar_stream stream);
 /* The schedule a call of this size takes on a device with `sms` SMs (host only, no device work; environment overrides
  * are not applied): CTA pairs or single CTAs, tile width, whether the K loop is cut across units (stream-K), how many
  * units (CTAs or pairs) work on how many tiles.  With `segments` != NULL also the work list of unit `unit` as

@@ -37,7 +37,10 @@
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <mutex>
+#include <optional>
+#include <vector>
 #include "../include/fp4ar.h"
 #include "../include/fp4ar_codec.cuh"
 #include "../include/fp4ar_async.cuh"
@@ -766,31 +769,141 @@ static StatusWords* gemm_status_word() {
   return p[dev];
 }
 
-// Partial accumulators of the stream-K split: one slot of 128 x 256 floats and four flags per SM, allocated at the
-// first call on a device and kept (19 MB on a B200).  Launches that share a device take turns on a slot through its
-// flags: a producer waits until the consumer of the previous launch has reset them.
-struct StreamKSpace { float* partial; uint32_t* flags; int slots; };
-static StreamKSpace g_stream_k_space[64] = {};
-static std::mutex g_stream_k_mu;
-static bool stream_k_space(int slots, StreamKSpace* out) {
-  StreamKSpace* sp = g_stream_k_space;
-  std::mutex& mu = g_stream_k_mu;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-  std::lock_guard<std::mutex> g(mu);
-  if (!sp[dev].partial) {
-    float* part = nullptr;
-    uint32_t* fl = nullptr;
-    const size_t pbytes = (size_t)slots * kBM * 256 * sizeof(float), fbytes = (size_t)slots * 4 * sizeof(uint32_t);
-    if (cudaMalloc(&part, pbytes) != cudaSuccess) { cudaGetLastError(); return false; }
-    if (cudaMalloc(&fl, fbytes) != cudaSuccess) { cudaGetLastError(); cudaFree(part); return false; }
-    if (cudaMemset(fl, 0, fbytes) != cudaSuccess) { cudaGetLastError(); cudaFree(part); cudaFree(fl); return false; }
-    sp[dev] = StreamKSpace{part, fl, slots};
+// Zeroed device memory, also while a stream of this thread is being captured (the allocation is not part of the graph).
+static void* alloc_zeroed(size_t bytes) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return nullptr;
+  void* p = nullptr;
+  cudaStream_t s = nullptr;
+  bool ok = cudaMalloc(&p, bytes) == cudaSuccess && cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess &&
+            cudaMemsetAsync(p, 0, bytes, s) == cudaSuccess && cudaStreamSynchronize(s) == cudaSuccess;
+  if (s) cudaStreamDestroy(s);
+  if (!ok) {
+    cudaGetLastError();
+    if (p) cudaFree(p);
+    p = nullptr;
   }
-  if (sp[dev].slots < slots) return false;
-  *out = sp[dev];
-  return true;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return p;
 }
+
+// Workspaces of the stream-K split: one slot of 128 x 256 floats and four flags per SM (19 MB on a B200).  A flag says that
+// a partial is there, not whose it is, so two launches that may run at the same time never share a workspace:
+//   - the launches of a stream follow one another and share one (streams are told apart by their id, which is never used
+//     again).  The first kSpaces streams of a device have their own; the launches of all later ones take turns on one
+//     more, by an event;
+//   - the launches that one capture records on one stream share one that their graph owns: the replays of a graph follow
+//     one another.  It can serve another graph once that one and its instances are gone.
+// Memory is allocated when it is first needed and kept; fp4ar_gemm_reset gives back what no graph owns.
+struct StreamKSpace {
+  void* mem = nullptr;                   // partials, then flags
+  unsigned long long stream = 0, capture = 0;
+  bool graph_owned = false;
+  std::atomic<bool> idle{false};         // set when the owning graph is gone, from a thread of CUDA: nothing else happens there
+};
+struct StreamKPool {
+  std::vector<std::unique_ptr<StreamKSpace>> spaces;
+  std::unique_ptr<StreamKSpace> shared;  // of the streams beyond kSpaces
+  cudaEvent_t turn = nullptr;            // its last launch
+};
+constexpr int kSpaces = 8;
+static StreamKPool* const g_stream_k = new StreamKPool[64];      // never destroyed: a graph may be released while the process ends
+static std::mutex g_stream_k_mu;
+static size_t stream_k_partial_bytes() { return (size_t)device_sm_count() * kBM * 256 * sizeof(float); }
+static size_t stream_k_flag_bytes() { return (size_t)device_sm_count() * 4 * sizeof(uint32_t); }
+
+// The workspace of one launch, held until the launch is enqueued.
+class StreamKLease {
+ public:
+  explicit StreamKLease(cudaStream_t stream) : lock_(g_stream_k_mu), stream_(stream) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+    StreamKPool& pool = g_stream_k[dev];
+    cudaStreamCaptureStatus status;
+    unsigned long long id = 0, capture = 0;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamGetCaptureInfo(stream, &status, &capture, &graph) != cudaSuccess) { cudaGetLastError(); return; }
+    const bool recording = status == cudaStreamCaptureStatusActive;
+    if (recording) id = (unsigned long long)(uintptr_t)stream;             // the id cannot be asked for during a capture
+    else if (status != cudaStreamCaptureStatusNone || cudaStreamGetId(stream, &id) != cudaSuccess) { cudaGetLastError(); return; }
+    StreamKSpace* free_one = nullptr;
+    int streams = 0;
+    for (auto& s : pool.spaces) {
+      if (s->graph_owned && s->idle.load(std::memory_order_acquire)) free_one = s.get();
+      else if (s->graph_owned == recording && s->stream == id && (!recording || s->capture == capture)) { space_ = s.get(); return; }
+      else if (!s->graph_owned) streams++;
+    }
+    if (recording) {
+      StreamKSpace* s = free_one ? free_one : add(pool);
+      if (!s || !zero_flags(s) || !give_to(graph, s)) return;
+      s->stream = id; s->capture = capture;
+      space_ = s;
+    } else if (streams < kSpaces) {
+      StreamKSpace* s = add(pool);
+      if (!s) return;
+      s->stream = id;
+      space_ = s;
+    } else {
+      if (!pool.turn && cudaEventCreateWithFlags(&pool.turn, cudaEventDisableTiming) != cudaSuccess) { cudaGetLastError(); return; }
+      if (!pool.shared) pool.shared = make();
+      if (!pool.shared || cudaStreamWaitEvent(stream, pool.turn, 0) != cudaSuccess) { cudaGetLastError(); return; }
+      space_ = pool.shared.get();
+      turn_ = pool.turn;
+    }
+  }
+  ~StreamKLease() {
+    if (turn_ && cudaEventRecord(turn_, stream_) != cudaSuccess) cudaGetLastError();
+  }
+  explicit operator bool() const { return space_ != nullptr; }
+  float* partial() const { return (float*)space_->mem; }
+  uint32_t* flags() const { return (uint32_t*)((char*)space_->mem + stream_k_partial_bytes()); }
+
+ private:
+  static std::unique_ptr<StreamKSpace> make() {
+    std::unique_ptr<StreamKSpace> s(new StreamKSpace);
+    s->mem = alloc_zeroed(stream_k_partial_bytes() + stream_k_flag_bytes());
+    if (!s->mem) s.reset();
+    return s;
+  }
+  static StreamKSpace* add(StreamKPool& pool) {
+    auto s = make();
+    if (!s) return nullptr;
+    pool.spaces.push_back(std::move(s));
+    return pool.spaces.back().get();
+  }
+  // A graph that ended in a launch which gave up may have left flags behind.
+  static bool zero_flags(StreamKSpace* s) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return false;
+    cudaStream_t st = nullptr;
+    const bool ok = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess &&
+                    cudaMemsetAsync((char*)s->mem + stream_k_partial_bytes(), 0, stream_k_flag_bytes(), st) == cudaSuccess &&
+                    cudaStreamSynchronize(st) == cudaSuccess;
+    if (st) cudaStreamDestroy(st);
+    if (!ok) cudaGetLastError();
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return ok;
+  }
+  static void CUDART_CB released(void* p) { static_cast<StreamKSpace*>(p)->idle.store(true, std::memory_order_release); }
+  static bool give_to(cudaGraph_t graph, StreamKSpace* s) {
+    s->graph_owned = true;
+    s->idle.store(false, std::memory_order_release);
+    cudaUserObject_t object;
+    if (cudaUserObjectCreate(&object, s, released, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+      cudaGetLastError();
+      s->idle.store(true, std::memory_order_release);
+      return false;
+    }
+    if (cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove) == cudaSuccess) return true;
+    cudaGetLastError();
+    cudaUserObjectRelease(object, 1);
+    return false;
+  }
+  std::lock_guard<std::mutex> lock_;
+  cudaStream_t stream_;
+  StreamKSpace* space_ = nullptr;
+  cudaEvent_t turn_ = nullptr;
+};
 
 }  // namespace fp4ar
 
@@ -962,9 +1075,10 @@ extern "C" int fp4ar_gemm_nvfp4(const fp4ar_push_view* push, int two_shot, const
   p.status = gemm_status_word();
   if (!p.status) return cuda_fail();
   p.timeout_ns = 2000000000ull;
+  std::optional<StreamKLease> lease;
   if (stream_k) {
-    StreamKSpace sp;
-    if (stream_k_space(device_sm_count(), &sp)) { p.stream_k = 1; p.sk_partial = sp.partial; p.sk_flags = sp.flags; }
+    lease.emplace((cudaStream_t)stream);
+    if (*lease) { p.stream_k = 1; p.sk_partial = lease->partial(); p.sk_flags = lease->flags(); }
   }
   CUtensorMap ma, mb;
   if (pl.narrow) {
@@ -1011,13 +1125,27 @@ extern "C" int fp4ar_gemm_reset(void) {
   StatusWords* s = gemm_status_word();
   if (!s) return cuda_fail();
   if (cudaMemset(s, 0, sizeof(StatusWords)) != cudaSuccess) return cuda_fail();
-  {
-    std::lock_guard<std::mutex> g(g_stream_k_mu);
-    const StreamKSpace& sp = g_stream_k_space[dev];
-    if (sp.flags && cudaMemset(sp.flags, 0, (size_t)sp.slots * 4 * sizeof(uint32_t)) != cudaSuccess) return cuda_fail();
+  std::lock_guard<std::mutex> g(g_stream_k_mu);
+  if (cudaDeviceSynchronize() != cudaSuccess) return cuda_fail();     // what was enqueued before the lock was taken
+  StreamKPool& pool = g_stream_k[dev];
+  std::vector<std::unique_ptr<StreamKSpace>> kept;
+  for (auto& s : pool.spaces) {
+    if (s->graph_owned && !s->idle.load(std::memory_order_acquire)) {
+      if (cudaMemset((char*)s->mem + stream_k_partial_bytes(), 0, stream_k_flag_bytes()) != cudaSuccess) return cuda_fail();
+      kept.push_back(std::move(s));
+    } else {
+      cudaFree(s->mem);
+    }
   }
+  pool.spaces.swap(kept);
+  if (pool.shared) { cudaFree(pool.shared->mem); pool.shared.reset(); }
   if (cudaDeviceSynchronize() != cudaSuccess) return cuda_fail();
   return FP4AR_OK;
+}
+
+extern "C" const void* fp4ar_gemm_workspace(fp4ar_stream stream) {
+  const StreamKLease lease((cudaStream_t)stream);
+  return lease ? lease.partial() : nullptr;
 }
 
 extern "C" int fp4ar_gemm_status(fp4ar_status_words* out) {

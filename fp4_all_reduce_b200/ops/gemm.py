@@ -90,8 +90,14 @@ def gemm_status() -> N.StatusWords:
 
 def gemm_reset() -> None:
     """After a GEMM whose status is not 0: synchronise, clear the status block and the hand-off flags of the partial
-    tiles, so that later launches do not wait on what the failed one left behind."""
+    tiles, so that later launches do not wait on what the failed one left behind.  Frees the workspaces of partial tiles
+    that no CUDA graph owns."""
     N.check(N.cuda().fp4ar_gemm_reset(), "fp4ar_gemm_reset")
+
+
+def gemm_workspace() -> int:
+    """Address of the workspace of partial tiles that a GEMM with a cut K loop takes on the current stream."""
+    return N.cuda().fp4ar_gemm_workspace(_stream()) or 0
 
 
 def gemm_plan(M: int, Nn: int, K: int, sms: int = 148, unit: Optional[int] = None):

@@ -159,3 +159,81 @@ def test_gemm_of_few_rows_equals_the_wide_tiles(M, K, Nn, monkeypatch):
     assert np.count_nonzero(q.cpu().numpy() != O.encode_static_f32(acc.cpu().numpy(), gs)) == 0
     assert torch.equal(q, q2)
     assert torch.equal(acc, wide_acc) and torch.equal(q, wide)
+
+
+def _captured_gemm(x, wt, gs, out, stream):
+    """A graph of one GEMM and the workspace that its launch took."""
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=stream):
+        G.gemm_nvfp4(x, wt, gs, out=out)
+        space = G.gemm_workspace()
+    return g, space
+
+
+def test_split_gemms_that_may_overlap_have_a_workspace_each(monkeypatch):
+    monkeypatch.setenv("FP4AR_GEMM_STREAM_K", "1")
+    torch.cuda.synchronize()
+    G.gemm_reset()
+    streams = [torch.cuda.Stream() for _ in range(11)]
+    spaces = []
+    for _ in range(2):
+        for s in streams:
+            with torch.cuda.stream(s):
+                spaces.append(G.gemm_workspace())
+    assert 0 not in spaces and spaces[:11] == spaces[11:]
+    assert len(set(spaces[:8])) == 8 and len(set(spaces[8:11])) == 1 and spaces[8] not in spaces[:8]
+    x, wt = _xw(1024, 512, N.HIDDEN, 0)
+    gs = G.calibrate_gs(x, wt)
+    out = torch.empty(1024, N.QROW_BYTES, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    kept = [_captured_gemm(x, wt, gs, out, streams[0]) for _ in range(3)]
+    owned = [space for _, space in kept]
+    assert len(set(owned)) == 3 and not set(owned) & set(spaces)
+    with torch.cuda.stream(streams[0]):
+        assert G.gemm_workspace() == spaces[0]
+    seen = set()
+    for _ in range(20):                                    # what a graph owned serves another one when it is gone
+        g, space = _captured_gemm(x, wt, gs, out, streams[1])
+        assert space not in owned
+        seen.add(space)
+        del g
+        torch.cuda.synchronize()
+    assert len(seen) < 20
+    del kept
+    torch.cuda.synchronize()
+    G.gemm_reset()
+
+
+def test_split_gemms_on_many_streams_at_once(monkeypatch):
+    """Launches of different inputs on eleven streams (three of them take turns on one workspace) and in graphs replayed on
+    others, nothing between them: every result equals the one computed alone."""
+    monkeypatch.setenv("FP4AR_GEMM_STREAM_K", "1")
+    G.gemm_reset()
+    M, K, n = 1024, 1024, 13
+    data, alone, outs = [], [], []
+    for i in range(n):
+        x, wt = _xw(M, K, N.HIDDEN, 20 + i)
+        gs = G.calibrate_gs(x, wt)
+        data.append((x, wt, gs))
+        alone.append(G.gemm_nvfp4(x, wt, gs).clone())
+        outs.append([torch.zeros_like(alone[0]) for _ in range(3)])
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(n)]
+    graphs = {i: _captured_gemm(*data[i], outs[i][0], streams[i])[0] for i in (11, 12)}
+    for rep in range(3):
+        for i, (x, wt, gs) in enumerate(data):
+            with torch.cuda.stream(streams[i]):
+                if i in graphs:
+                    outs[i][0].zero_()
+                    graphs[i].replay()
+                    outs[i][rep].copy_(outs[i][0])
+                else:
+                    G.gemm_nvfp4(x, wt, gs, out=outs[i][rep])
+    torch.cuda.synchronize()
+    assert G.gemm_status().code == 0
+    for i in range(n):
+        for o in outs[i]:
+            assert torch.equal(o, alone[i]), i
+    graphs.clear()
+    torch.cuda.synchronize()
+    G.gemm_reset()

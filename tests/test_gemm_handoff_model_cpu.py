@@ -13,3 +13,9 @@ def test_product_rules_are_safe(units, launches):
 @pytest.mark.parametrize("variant", ["no_free_wait", "early_reset"])
 def test_a_missing_rule_is_caught(variant):
     assert M.check(6, 6, seeds=150, variant=variant) > 0
+
+
+@pytest.mark.parametrize("units,streams", [(2, 2), (5, 2), (5, 3)])
+def test_launches_of_several_streams_need_a_workspace_each(units, streams):
+    assert M.check(units, 2 * streams, seeds=150, streams=streams) == 0
+    assert M.check(units, 2 * streams, seeds=150, streams=streams, variant="one_space") > 0
