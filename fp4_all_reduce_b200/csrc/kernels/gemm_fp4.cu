@@ -758,17 +758,6 @@ static bool make_map_3d(CUtensorMap* m, const void* base, int rows, int k, int b
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-static StatusWords* gemm_status_word() {
-  static StatusWords* p[64] = {nullptr};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  if (!p[dev]) {
-    if (cudaMalloc(&p[dev], sizeof(StatusWords)) != cudaSuccess) return nullptr;
-    cudaMemset(p[dev], 0, sizeof(StatusWords));
-  }
-  return p[dev];
-}
-
 // Zeroed device memory, also while a stream of this thread is being captured (the allocation is not part of the graph).
 static void* alloc_zeroed(size_t bytes) {
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
@@ -784,6 +773,24 @@ static void* alloc_zeroed(size_t bytes) {
     p = nullptr;
   }
   cudaThreadExchangeStreamCaptureMode(&mode);
+  return p;
+}
+
+// The status block of a device, allocated by the first thread that needs it.
+static StatusWords* gemm_status_word() {
+  static std::atomic<StatusWords*> words[64];
+  static std::mutex mu;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  StatusWords* p = words[dev].load(std::memory_order_acquire);
+  if (!p) {
+    std::lock_guard<std::mutex> g(mu);
+    p = words[dev].load(std::memory_order_acquire);
+    if (!p) {
+      p = (StatusWords*)alloc_zeroed(sizeof(StatusWords));
+      words[dev].store(p, std::memory_order_release);
+    }
+  }
   return p;
 }
 

@@ -1,6 +1,10 @@
 """The tcgen05 GEMM with NVFP4 epilogue: accumulators against an FP32 matmul, quantised rows bit for bit
 against the host quantiser applied to the kernel's own accumulators, and the fused GEMM -> push -> AllReduce
 path on emulated ranks against the host model fed with the kernel's NVFP4 partials."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -237,3 +241,26 @@ def test_split_gemms_on_many_streams_at_once(monkeypatch):
     graphs.clear()
     torch.cuda.synchronize()
     G.gemm_reset()
+
+
+@pytest.mark.parametrize("M", [16, 1024])
+def test_first_gemm_of_a_process_may_be_captured(M):
+    """Nothing that the first call sets up (status block, workspace, shared-memory limits) needs a call outside the capture."""
+    code = f"""
+import torch
+from fp4_all_reduce_b200.ops import gemm as G
+x = torch.randn({M}, 2048, device="cuda").to(torch.bfloat16)
+wt = torch.randn(6144, 2048, device="cuda").to(torch.bfloat16)
+out = torch.zeros({M}, 3456, dtype=torch.uint8, device="cuda")
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    G.gemm_nvfp4(x, wt, 0.05, out=out)
+g.replay()
+torch.cuda.synchronize()
+assert G.gemm_status().code == 0 and torch.equal(out, G.gemm_nvfp4(x, wt, 0.05)) and out.any()
+"""
+    env = dict(os.environ, FP4AR_GEMM_STREAM_K="1") if M > 384 else dict(os.environ)
+    r = subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), env=env,
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
