@@ -240,6 +240,13 @@ __device__ __forceinline__ bool gemm_wait(uint64_t* bar, uint32_t parity, const 
   return true;
 }
 
+// A CTA that gives up may still have copies on their way into its shared memory and MMAs at work on its TMEM: it leaves only
+// when their barrier says that they are through (10 ms at most).
+__device__ __forceinline__ void gemm_settle(uint64_t* bar, uint32_t parity) {
+  const unsigned long long t0 = global_timer_ns();
+  while (!mbar_test(bar, parity) && global_timer_ns() - t0 < 10000000ull) {}
+}
+
 // Bounded wait until *flag == want (acquire); false when it gave up or the CTA is aborting.
 __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
   uint32_t v;
@@ -335,6 +342,8 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   uint64_t* acc_empty = acc_full + 2;                               // [2]
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile uint32_t* abort_flag = tmem_holder + 1;
+  uint64_t* settled = reinterpret_cast<uint64_t*>(tmem_holder + 2);
+  uint32_t issued = 0;                 // ring stages that this CTA's producer has filled
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_tiles = p.N / BN, m_tiles = (p.M + kBM * G - 1) / (kBM * G);
@@ -347,6 +356,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; s++) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
     for (int a = 0; a < 2; a++) { mbar_init(acc_full + a, 1); mbar_init(acc_empty + a, 128 * G); }
+    mbar_init(settled, 1);
     *abort_flag = 0u;
     mbar_init_fence();
   }
@@ -376,19 +386,8 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         for (int j = 0; j < sg.count; j++, it++) {
           const int kb = sg.lo + j;
           const int s = it % kStages;
-          if (!gemm_wait(empty + s, ((it / kStages) & 1u) ^ 1u, gw, 1)) {
-            // giving up: let the loads already issued land before the CTA (and its shared memory) goes away
-            if (leads) {
-              for (uint32_t back = 1; back <= (uint32_t)kStages && back <= it; back++) {
-                const uint32_t j = it - back;
-                uint32_t spins = 0;
-                while (!mbar_test(full + (j % kStages), (j / kStages) & 1u) && ++spins < (1u << 20)) {}
-              }
-            } else {
-              for (int w = 0; w < 2000; w++) __nanosleep(1000);   // its loads complete under the leader's barriers: 2 ms
-            }
-            goto done;
-          }
+          if (!gemm_wait(empty + s, ((it / kStages) & 1u) ^ 1u, gw, 1)) goto done;
+          issued = it + 1;
           if constexpr (G == 2) {
             // both CTAs' bytes are counted under the leader's barrier; only the leader announces them
             const uint32_t lead_full = cluster_addr(full + s, 0u);
@@ -566,6 +565,17 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 done:
   tc_fence_before();
   __syncthreads();
+  if (*abort_flag != 0u) {
+    if (leads && threadIdx.x == 0)
+      for (uint32_t i = issued > (uint32_t)kStages ? issued - kStages : 0u; i < issued; i++) gemm_settle(full + i % kStages, (i / kStages) & 1u);
+    if (!leads && threadIdx.x == 0)
+      for (int w = 0; w < 2000; w++) __nanosleep(1000);     // its loads complete under the leader's barriers: 2 ms
+    if (leads && threadIdx.x == 32) {
+      if constexpr (G == 2) umma_commit_pair(settled); else umma_commit(settled);
+      gemm_settle(settled, 0u);
+    }
+    __syncthreads();
+  }
   if constexpr (G == 2) cluster_sync_all();   // neither CTA frees TMEM or leaves while the other's MMAs, commits or arrivals may still touch it
   if (warp == 1) {
     __syncwarp();
@@ -611,6 +621,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   uint64_t* acc_full = empty + kNarrowStages;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile uint32_t* abort_flag = tmem_holder + 1;
+  int issued = 0;                      // ring stages filled
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m_tiles = (p.M + kBM - 1) / kBM, kblocks = p.K / kBK, trips = (kblocks + atoms - 1) / atoms;
@@ -637,14 +648,8 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   if (warp == 0) {
     if (lane == 0) {
       for (int it = 0, st = 0, round = 0; it < trips; it++) {
-        if (!gemm_wait(empty + st, (round & 1u) ^ 1u, gw, 1)) {
-          // giving up: let the loads already issued land before the CTA (and its shared memory) goes away
-          for (int back = 1; back <= stages && back <= it; back++) {
-            uint32_t spins = 0;
-            while (!mbar_test(full + ((it - back) % stages), ((it - back) / stages) & 1u) && ++spins < (1u << 20)) {}
-          }
-          break;
-        }
+        if (!gemm_wait(empty + st, (round & 1u) ^ 1u, gw, 1)) break;
+        issued = it + 1;
         mbar_arrive_expect(full + st, stage_bytes);
         if (atoms > 1) {
           tma_load_3d(ring + st * stage_bytes, &map_a, m0, it * atoms, full + st);
@@ -715,6 +720,12 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   }
   tc_fence_before();
   __syncthreads();
+  if (*abort_flag != 0u) {
+    if (threadIdx.x == 0)
+      for (int i = max(0, issued - stages); i < issued; i++) gemm_settle(full + i % stages, (i / stages) & 1);
+    if (threadIdx.x == 32) gemm_settle(acc_full, 0u);       // committed behind every MMA issued
+    __syncthreads();
+  }
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, kCols); }
 }
 

@@ -264,3 +264,37 @@ assert G.gemm_status().code == 0 and torch.equal(out, G.gemm_nvfp4(x, wt, 0.05))
     r = subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), env=env,
                        capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr
+
+
+class _Words:
+    """`n` 32-bit words of device memory at an address, for torch.as_tensor."""
+
+    def __init__(self, address, n):
+        self.__cuda_array_interface__ = {"shape": (n,), "typestr": "<i4", "data": (address, False), "version": 3}
+
+
+@pytest.mark.parametrize("pair", [0, 1])
+def test_a_hand_off_that_never_comes_ends_with_a_status(pair, monkeypatch):
+    """A flag that is neither "free" nor "written" lets the wait of its producer and of its consumer run out (2 s): the launch
+    reports it and ends, and after a reset the same call gives the same rows as before."""
+    monkeypatch.setenv("FP4AR_GEMM_STREAM_K", "1")
+    monkeypatch.setenv("FP4AR_GEMM_PAIR", str(pair))
+    x, wt = _xw(1024, 1024, N.HIDDEN, 4)
+    gs = G.calibrate_gs(x, wt)
+    good = G.gemm_nvfp4(x, wt, gs).clone()
+    torch.cuda.synchronize()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    flags = torch.as_tensor(_Words(G.gemm_workspace() + sms * 128 * 256 * 4, 4 * sms), device="cuda")
+    assert not flags.any()
+    unit = 8                                  # an even CTA: the leader where CTAs work in pairs
+    flags[4 * unit] = 2
+    G.gemm_nvfp4(x, wt, gs)
+    torch.cuda.synchronize()
+    st = G.gemm_status()
+    assert st.code == 2 and st.detail in (16 + 5, 16 + 6) and st.count >= 1
+    del flags
+    G.gemm_reset()
+    for _ in range(2):
+        assert torch.equal(G.gemm_nvfp4(x, wt, gs), good)
+    torch.cuda.synchronize()
+    assert G.gemm_status().code == 0
