@@ -296,6 +296,10 @@ __device__ __forceinline__ void pack32_bf16(const float* f, uint4* c) {
 __device__ __forceinline__ bool values_pending(uint4 q) {
   return (q.x == kSentWord) | (q.y == kSentWord) | (q.z == kSentWord) | (q.w == kSentWord);
 }
+// A word of eight -0 as eight +0, which a sum that starts at +0 cannot tell apart.
+__device__ __forceinline__ uint4 without_sentinel(uint4 q) {
+  return make_uint4(q.x == kSentWord ? 0u : q.x, q.y == kSentWord ? 0u : q.y, q.z == kSentWord ? 0u : q.z, q.w == kSentWord ? 0u : q.w);
+}
 __device__ __forceinline__ bool scales_pending(uint32_t sf2) { return (sf2 & 0x8080u) != 0; }
 __device__ __forceinline__ bool rowscale_pending(uint32_t bits) { return bits == kSentRow; }
 

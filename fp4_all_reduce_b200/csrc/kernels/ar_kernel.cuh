@@ -486,6 +486,11 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T, MT>::kMa
             bool pend = false;
 #pragma unroll
             for (int u = 0; u < kOwnBatch; u++) pend |= own_pending(wq[u], wsf[u], wrs[u]);
+            if (IN == 1 && pend) {     // the own contribution is the caller's row: eight -0 are eight zeros, nothing to wait for
+#pragma unroll
+              for (int u = 0; u < kOwnBatch; u++)
+                if (s0 + u == me) wq[u] = without_sentinel(wq[u]);
+            }
             if (MT == 0 && pend) {
               const unsigned long long t0 = global_timer_ns();
               uint32_t n = 0;

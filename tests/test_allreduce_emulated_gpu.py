@@ -5,12 +5,15 @@ Counterpart of the reference project's integration gate (harness/fp4ar_bench.cu:
 tests/negative_control.sh), which needs 2 or 4 GPUs; the multi-GPU form of this gate is
 tests/test_allreduce_multigpu.py.
 """
+import numpy as np
 import pytest
 import torch
 
 from fp4_all_reduce_b200 import _native as N
+from fp4_all_reduce_b200 import oracle as O
 from fp4_all_reduce_b200.harness.gate import CellConfig, gate_cell_emulated, make_inputs, Outputs, args_for, mismatches
-from fp4_all_reduce_b200.parallel.context import EmulatedGroup
+from fp4_all_reduce_b200.parallel.context import EmulatedGroup, make_args
+from fp4_all_reduce_b200.utils import data as D
 
 pytestmark = pytest.mark.gpu
 
@@ -154,4 +157,28 @@ def test_narrow_and_wide_shapes_at_their_limits(P, inp, epi):
             torch.cuda.synchronize()
             assert g.status(0).ok, g.status(0).describe()
             assert sum(mismatches(c, data, outs, r) for r in range(P)) == 0, c
+    g.close()
+
+
+@pytest.mark.parametrize("P", [4, 8])
+@pytest.mark.parametrize("rows", [30, 700])
+def test_own_rows_may_hold_what_the_window_calls_not_yet_written(P, rows):
+    """Two-shot, NVFP4 input: a rank's contribution to a row it owns never crosses a window, so a word of eight -0 there is
+    eight zeros and nothing to wait for, in the narrow build (30 rows) as in the wide one."""
+    dev = torch.device("cuda", 0)
+    q = [O.encode_static(O.bf16_bits(D.partial(rows, r)), 0.01) for r in range(P)]
+    for r in range(P):
+        q[r][r::P, 64:68] = 0
+    want = O.allreduce(q, algo=1, input_kind=1, gs=[0.01] * P)["out"]
+    xs = [torch.from_numpy(a.copy()).to(dev) for a in q]
+    for r in range(P):
+        xs[r][r::P, 64:68] = 0x88
+    outs = [torch.zeros(rows, N.HIDDEN, dtype=torch.bfloat16, device=dev) for _ in range(P)]
+    g = EmulatedGroup(P, rows)
+    g.set_timeout_ms(1000)
+    g.launch([make_args(x=xs[r], out=outs[r], rows=rows, input=N.IN_NVFP4, gs=[0.01] * P) for r in range(P)])
+    torch.cuda.synchronize()
+    assert g.status(0).ok, g.status(0).describe()
+    for r in range(P):
+        assert np.array_equal(O.bf16_bits(outs[r]), want), r
     g.close()
