@@ -133,6 +133,8 @@ def cuda() -> C.CDLL:
     ip = C.POINTER(C.c_int)
     lib.fp4ar_gemm_plan.argtypes = [C.c_int, C.c_int, C.c_int, C.c_int, ip, ip, ip, ip, ip, C.c_int, ip, C.c_int]
     lib.fp4ar_gemm_plan.restype = C.c_int
+    lib.fp4ar_launch_plan.argtypes = [C.c_int, C.c_int, C.POINTER(Args), C.POINTER(C.c_int)]
+    lib.fp4ar_launch_plan.restype = C.c_int
     lib.fp4ar_gemm_reset.argtypes = []
     lib.fp4ar_gemm_reset.restype = C.c_int
     lib.fp4ar_gemm_workspace.argtypes = [vp]

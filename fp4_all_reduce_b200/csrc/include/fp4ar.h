@@ -116,6 +116,9 @@ const char* fp4ar_last_cuda_error(void);
 const char* fp4ar_build_info(void);
 /* Teams per CTA of the compiled kernel for this shape (0 = not compiled). */
 int fp4ar_has_kernel(int nranks, int algo, int input, int epilogue, int team_warps);
+/* What a launch of these arguments takes (host only: hidden, pointers and scales are not looked at): team width in warps, teams
+ * per CTA, 1 for the narrow build of few rows, the two pipeline depths, bytes of shared memory. */
+int fp4ar_launch_plan(int nranks, int ctas_per_rank, const fp4ar_args* args, int* plan6);
 /* Warps per row team a launch uses when tune[2] is 0 (algo: FP4AR_ALGO_ONESHOT / TWOSHOT, already resolved). */
 int fp4ar_default_team_warps(int nranks, int algo);
 

@@ -72,6 +72,8 @@ struct ArParams {
   unsigned long long* phase_cycles;   // tuning builds only (-DFP4AR_PHASE_TIMERS): 16 per-phase cycle counters
 };
 
+constexpr int kSmemLimit = 227 * 1024;      // shared memory of a CTA on sm_100
+
 template <int P, int ALGO, int IN, int EPI, int T, int MT = 0>
 struct ArShape {
   static constexpr int NJ = 6 / T;                                   // pairs per lane per row
@@ -83,8 +85,13 @@ struct ArShape {
   // kMaxLag bounds them and sizes the record ring.
   static constexpr int kMaxLag = kTwoShot ? 4 : 1;
   // Row buffers, a ring over the rows in the order in which a team consumes them: x of step k, residual of step k, x of
-  // step k + 1, ...  Each is loaded a whole step before it is used.
-  static constexpr int NRB = IN == 0 ? (EPI > 0 ? 3 : 2) : (EPI > 0 ? 2 : 0);
+  // step k + 1, ...  Each is loaded a whole step before it is used.  Three-warp teams of four ranks have two buffers, one
+  // for x and one for the residual, each loaded again as soon as its row is done with: with three only three teams fit
+  // a CTA.  16384 / 4096 / 1024 rows, three buffers -> two: BF16 out 235 -> 219 / 65 -> 59 / 22.2 -> 19.9 us, NVFP4 276 -> 239 /
+  // 76 -> 66 / 26.0 -> 21.5, MXFP8 267 -> 230 / 73 -> 63 / 25.0 -> 20.9.  At eight ranks it is 20.7 for 22.9 us at 1024 rows but 241
+  // for 207 at 16384.
+  static constexpr bool kShortRing = IN == 0 && EPI > 0 && kTwoShot && T == 3 && P <= 4;
+  static constexpr int NRB = IN == 0 ? (EPI > 0 && !kShortRing ? 3 : 2) : (EPI > 0 ? 2 : 0);
   static constexpr int NREC = (IN == 1 ? 2 : 1) + kMaxLag;
   static constexpr int kOutBytes = EPI <= 1 ? kRowBytes : (EPI == 2 ? 3584 : 6400);
   static constexpr int kMisc = 128;                                  // mbarriers + reduction scratch
@@ -95,9 +102,11 @@ struct ArShape {
   // residual: those shapes get fewer, fatter threads.
   // (Register budget per thread = 65536 / (32 * T * kMaxTeams).)
   static constexpr int kHeavy = (ALGO == 1 || EPI > 0) ? 1 : 0;
-  // Three-warp teams: 4 per CTA (heavy shapes) or 5; six-warp teams: 3 per CTA (18 warps at up to 112 registers; a
-  // fourth team at 80 registers measured 20-30 % slower).
-  static constexpr int kMaxTeams = MT > 0 ? MT : (T == 3 ? (kHeavy ? 4 : 5) : 3);
+  // Three-warp teams: 4 per CTA (heavy shapes) or 5, as far as they fit into shared memory; six-warp teams: 3 per CTA
+  // (18 warps at up to 112 registers; a fourth team at 80 registers measured 20-30 % slower).
+  static constexpr int kWantTeams = MT > 0 ? MT : (T == 3 ? (kHeavy ? 4 : 5) : 3);
+  static constexpr int kFitTeams = (kSmemLimit - kCtaExtra) / kTeamBytes;
+  static constexpr int kMaxTeams = kFitTeams < kWantTeams ? kFitTeams : kWantTeams;
   static __host__ __device__ constexpr int smem_bytes(int teams) { return teams * kTeamBytes + kCtaExtra; }
 };
 
@@ -224,7 +233,7 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T, MT>::kMa
   if (leader && nk > 0) {
     if (IN == 0) {
       load_row(x_item(0), io.x, row_of(0));
-      if (nk > 1) load_row(x_item(1), io.x, row_of(1));
+      if (nk > 1 && !S::kShortRing) load_row(x_item(1), io.x, row_of(1));
     } else if (IN == 1) {
       mbar_arrive_expect(qbar + 0, kQRowBytes);
       bulk_load(recs, io.x + (size_t)row_of(0) * kQRowBytes, kQRowBytes, qbar + 0);
@@ -429,7 +438,10 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T, MT>::kMa
     tsync.sync();
     FP4AR_PHASE(1);   // drain wait + barrier
     if (EPI > 0 && leader) {                    // the buffer of the residual that left in the previous step is free
-      if (IN == 0) {
+      if (S::kShortRing) {
+        const int kr = k - lag_f;
+        if (kr >= 0 && kr < nk) load_row(res_item(k), io.res_in, row_of(kr));
+      } else if (IN == 0) {
         if (k > 0 && k + 1 < nk) load_row(x_item(k + 1), io.x, row_of(k + 1));
       } else {
         const int kr = k + 1 - lag_f;
@@ -744,7 +756,9 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T, MT>::kMa
       for (int s = tw; s < P; s += T)
         if (s != me) bulk_store(my_buf() + rs_slot(s, row_of(k)), recs + (k % NREC) * kRecStride, IN == 0 ? (uint32_t)kRecPayload : (uint32_t)kQRowBytes);
     }
-    if (IN == 0 && EPI > 0 && leader) {         // into the buffer of the row just encoded
+    if (S::kShortRing) {
+      if (leader && k + 1 < nk) load_row(x_item(k + 1), io.x, row_of(k + 1));
+    } else if (IN == 0 && EPI > 0 && leader) {         // into the buffer of the row just encoded
       const int kr = k + 1 - lag_f;
       if (kr >= 0 && kr < nk) load_row(res_item(k + 1), io.res_in, row_of(kr));
     }

@@ -279,6 +279,69 @@ extern "C" const char* fp4ar_build_info(void) {
 
 static bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
+// The kernel, team count, pipeline depths and shared memory of one call.
+struct LaunchPlan {
+  const ArKernelEntry* ke;
+  int algo, teams, lag_owner, lag_finish, smem;
+};
+static int plan_launch(const fp4ar_args& a0, int nranks, int ctas_per_rank, int smem_optin, LaunchPlan* pl) {
+  int algo = a0.algo;
+  if (algo == FP4AR_ALGO_AUTO) algo = nranks <= 2 ? FP4AR_ALGO_ONESHOT : FP4AR_ALGO_TWOSHOT;
+  if (algo != FP4AR_ALGO_ONESHOT && algo != FP4AR_ALGO_TWOSHOT) return FP4AR_ERR_ARGUMENT;
+  if (nranks == 1) algo = FP4AR_ALGO_ONESHOT;
+  const int width = team_warps_for(a0, nranks, algo);
+  const ArKernelEntry* ke = find_kernel(nranks, algo, a0.input, a0.epilogue, width);
+  // a team width that comes from the environment is a preference: shapes not compiled at that width use their default
+  if (!ke && a0.tune[2] <= 0) ke = find_kernel(nranks, algo, a0.input, a0.epilogue, default_team_warps(nranks, algo));
+  if (!ke) return FP4AR_ERR_UNSUPPORTED;
+  // Few rows per CTA: the narrow build (six-warp teams, at most two per CTA) where its two teams need no more trips than
+  // the teams of the wide one.  A call of that size is one row's latency, and half as many pairs per lane, no spills and
+  // every source of an owned row in flight at once shorten it.  Block, BF16 in, one team trip, wide -> narrow: two ranks
+  // 5.2 -> 4.2 us, four 6.6 -> 6.2, eight 9.6 -> 9.2 (NVFP4 in 8.3 -> 7.0).  A call that names a width or a team count
+  // gets what it names.
+  const int rows_per_cta = (a0.rows + ctas_per_rank - 1) / ctas_per_rank;
+  if (a0.tune[0] <= 0 && a0.tune[2] <= 0 && ke->T == default_team_warps(nranks, algo)) {
+    const ArKernelEntry* ne = find_kernel(nranks, algo, a0.input, a0.epilogue, 6, true);
+    auto trips = [&](int teams) { return (rows_per_cta + teams - 1) / teams; };
+    if (ne && trips(ne->max_teams) <= trips(ke->max_teams)) ke = ne;
+  }
+  int teams = ke->max_teams;
+  const int fit = (smem_optin - ke->cta_extra) / ke->team_bytes;
+  if (fit < teams) teams = fit;
+  if (a0.tune[0] > 0 && a0.tune[0] < teams) teams = a0.tune[0];
+  if (rows_per_cta < teams) teams = rows_per_cta;      // a smaller CTA starts sooner
+  if (teams < 1) return FP4AR_ERR_UNSUPPORTED;
+  // Two-shot pipeline depths: tune[3] = lag_owner | lag_finish << 4 when set, otherwise by team width and degree.
+  // Three-warp teams (measured on 4 and 8 GPUs): (1,2) at four ranks, where the kernel is bound by its own codec work
+  // at large row counts and the shallow pipeline wins; (2,3) at eight, where every row waits on seven peers and one
+  // more step of slack at each hand-off pays at every row count (16K rows: 284 -> 228 us).  A step of a six-warp team
+  // takes about half as long, so those shapes run (2,3) everywhere.  Eight GPUs, 16384 rows, AR / block: (2,3) 179 /
+  // 238 us, (2,4) 192 / 240, (3,4) 181 / 240; 1024 rows: 24.6, 27.6, 23.2 us.  Four GPUs, 16384 rows: (1,2) 209 / 231,
+  // (2,3) 150 / 199, (2,4) 156 / 202, (3,4) 154 / 201; 1024 rows: 23.6, 17.8, 18.8, 18.6 us.
+  {
+    int lo = a0.tune[3] & 15, lf = (a0.tune[3] >> 4) & 15;
+    if (lo < 1 || lf <= lo || lf > 4) {
+      if (rows_per_cta <= teams) { lo = 1; lf = 2; }     // one row per team: nothing to overlap, a deeper pipeline only adds steps
+      else if (ke->T == 6 || nranks >= 6) { lo = 2; lf = 3; }
+      else { lo = 1; lf = 2; }
+    }
+    pl->lag_owner = lo; pl->lag_finish = lf;
+  }
+  pl->ke = ke; pl->algo = algo; pl->teams = teams;
+  pl->smem = teams * ke->team_bytes + ke->cta_extra;
+  return FP4AR_OK;
+}
+
+extern "C" int fp4ar_launch_plan(int nranks, int ctas_per_rank, const fp4ar_args* args, int* plan6) {
+  if (!args || !plan6 || nranks < 1 || ctas_per_rank < 1 || args->rows < 1) return FP4AR_ERR_ARGUMENT;
+  LaunchPlan pl;
+  const int rc = plan_launch(*args, nranks, ctas_per_rank, kSmemLimit, &pl);
+  if (rc != FP4AR_OK) return rc;
+  plan6[0] = pl.ke->T; plan6[1] = pl.teams; plan6[2] = pl.ke->narrow; plan6[3] = pl.lag_owner; plan6[4] = pl.lag_finish;
+  plan6[5] = pl.smem;
+  return FP4AR_OK;
+}
+
 extern "C" int fp4ar_launch(fp4ar_ctx* c, const fp4ar_args* args, fp4ar_stream stream) {
   if (!c || !args) return FP4AR_ERR_ARGUMENT;
   const fp4ar_args& a0 = args[0];
@@ -291,32 +354,13 @@ extern "C" int fp4ar_launch(fp4ar_ctx* c, const fp4ar_args* args, fp4ar_stream s
   if (*reinterpret_cast<volatile uint32_t*>(c->poison_host) != 0u) return FP4AR_ERR_POISONED;
   // Nothing to reduce: no launch, so the device call counter (and with it the buffer parity) does not move.
   if (a0.rows == 0) return FP4AR_OK;
-  int algo = a0.algo;
-  if (algo == FP4AR_ALGO_AUTO) algo = c->nranks <= 2 ? FP4AR_ALGO_ONESHOT : FP4AR_ALGO_TWOSHOT;
-  if (algo != FP4AR_ALGO_ONESHOT && algo != FP4AR_ALGO_TWOSHOT) return FP4AR_ERR_ARGUMENT;
-  if (c->nranks == 1) algo = FP4AR_ALGO_ONESHOT;
-  const int width = team_warps_for(a0, c->nranks, algo);
-  const ArKernelEntry* ke = find_kernel(c->nranks, algo, a0.input, a0.epilogue, width);
-  // a team width that comes from the environment is a preference: shapes not compiled at that width use their default
-  if (!ke && a0.tune[2] <= 0) ke = find_kernel(c->nranks, algo, a0.input, a0.epilogue, default_team_warps(c->nranks, algo));
-  if (!ke) return FP4AR_ERR_UNSUPPORTED;
-  // Few rows per CTA: the narrow build (six-warp teams, at most two per CTA) where its two teams need no more trips than
-  // the teams of the wide one.  A call of that size is one row's latency, and half as many pairs per lane, no spills and
-  // every source of an owned row in flight at once shorten it.  Block, BF16 in, one team trip, wide -> narrow: two ranks
-  // 5.2 -> 4.2 us, four 6.6 -> 6.2, eight 9.6 -> 9.2 (NVFP4 in 8.3 -> 7.0).  A call that names a width or a team count
-  // gets what it names.
-  const int rows_per_cta = (a0.rows + c->ctas_per_rank - 1) / c->ctas_per_rank;
-  if (a0.tune[0] <= 0 && a0.tune[2] <= 0 && ke->T == default_team_warps(c->nranks, algo)) {
-    const ArKernelEntry* ne = find_kernel(c->nranks, algo, a0.input, a0.epilogue, 6, true);
-    auto trips = [&](int teams) { return (rows_per_cta + teams - 1) / teams; };
-    if (ne && trips(ne->max_teams) <= trips(ke->max_teams)) ke = ne;
+  LaunchPlan pl;
+  {
+    const int rc = plan_launch(a0, c->nranks, c->ctas_per_rank, c->max_smem_optin, &pl);
+    if (rc != FP4AR_OK) return rc;
   }
-  int teams = ke->max_teams;
-  const int fit = (c->max_smem_optin - ke->cta_extra) / ke->team_bytes;
-  if (fit < teams) teams = fit;
-  if (a0.tune[0] > 0 && a0.tune[0] < teams) teams = a0.tune[0];
-  if (rows_per_cta < teams) teams = rows_per_cta;      // a smaller CTA starts sooner
-  if (teams < 1) return FP4AR_ERR_UNSUPPORTED;
+  const ArKernelEntry* ke = pl.ke;
+  const int algo = pl.algo, teams = pl.teams, smem = pl.smem;
 
   ArParams prm;
   std::memset(&prm, 0, sizeof(prm));
@@ -354,22 +398,7 @@ extern "C" int fp4ar_launch(fp4ar_ctx* c, const fp4ar_args* args, fp4ar_stream s
   prm.cap = c->geo.cap; prm.capo = c->geo.capo;
   prm.rs_stride = (unsigned long long)c->geo.capo * kRecStride;
   prm.buf_bytes = c->geo.buf_bytes; prm.timeout_ns = c->timeout_ns;
-  // Two-shot pipeline depths: tune[3] = lag_owner | lag_finish << 4 when set, otherwise by team width and degree.
-  // Three-warp teams (measured on 4 and 8 GPUs): (1,2) at four ranks, where the kernel is bound by its own codec work
-  // at large row counts and the shallow pipeline wins; (2,3) at eight, where every row waits on seven peers and one
-  // more step of slack at each hand-off pays at every row count (16K rows: 284 -> 228 us).  A step of a six-warp team
-  // takes about half as long, so those shapes run (2,3) everywhere.  Eight GPUs, 16384 rows, AR / block: (2,3) 179 /
-  // 238 us, (2,4) 192 / 240, (3,4) 181 / 240; 1024 rows: 24.6, 27.6, 23.2 us.  Four GPUs, 16384 rows: (1,2) 209 / 231,
-  // (2,3) 150 / 199, (2,4) 156 / 202, (3,4) 154 / 201; 1024 rows: 23.6, 17.8, 18.8, 18.6 us.
-  {
-    int lo = a0.tune[3] & 15, lf = (a0.tune[3] >> 4) & 15;
-    if (lo < 1 || lf <= lo || lf > 4) {
-      if (rows_per_cta <= teams) { lo = 1; lf = 2; }     // one row per team: nothing to overlap, a deeper pipeline only adds steps
-      else if (ke->T == 6 || c->nranks >= 6) { lo = 2; lf = 3; }
-      else { lo = 1; lf = 2; }
-    }
-    prm.lag_owner = lo; prm.lag_finish = lf;
-  }
+  prm.lag_owner = pl.lag_owner; prm.lag_finish = pl.lag_finish;
 #ifdef FP4AR_PHASE_TIMERS
   prm.phase_cycles = phase_buffer();
 #endif
@@ -382,7 +411,6 @@ extern "C" int fp4ar_launch(fp4ar_ctx* c, const fp4ar_args* args, fp4ar_stream s
     if (last > c->geo.buf_bytes || 2 * c->geo.buf_bytes > c->window_bytes) return FP4AR_ERR_ARGUMENT;
   }
 
-  const int smem = teams * ke->team_bytes + ke->cta_extra;
   {
     // the limit is raised once per (context, kernel), not on every launch
     std::lock_guard<std::mutex> lk(c->mu);

@@ -137,6 +137,15 @@ class EmulatedGroup(_Base):
         N.check(N.cuda().fp4ar_reset(self._ctx), "fp4ar_reset")
 
 
+def launch_plan(nranks: int, rows: int, *, ctas_per_rank: int = 148, **kw) -> dict:
+    """What a call of `rows` rows takes (host only; `kw` as for `make_args`): team width, teams per CTA, narrow build or
+    not, the two-shot pipeline depths, shared memory."""
+    a = make_args(x=None, out=None, rows=rows, **kw)
+    v = (C.c_int * 6)()
+    N.check(N.cuda().fp4ar_launch_plan(nranks, ctas_per_rank, C.byref(a), v), "fp4ar_launch_plan")
+    return dict(zip(("team_warps", "teams", "narrow", "lag_owner", "lag_finish", "smem"), v))
+
+
 def input_sets_for(rows: int, row_bytes: int, l2_bytes: int = 126 * 1024 * 1024, most: int = 24) -> int:
     """How many rotating copies of a [rows, row_bytes] input a timed chain needs so that consecutive calls never find
     their input in the L2 cache (together they exceed twice its size)."""

@@ -163,3 +163,24 @@ def test_a_flag_without_a_truth_value_raises_its_own_error(front):
         front.add_rmsnorm(x, x, w, 1e-6, 1.0, 1, 1.0, torch.ones(2), None)
     with pytest.raises(RuntimeError, match="ambiguous"):
         front.gemm(x, x, 1.0, torch.ones(2), None)
+
+
+def test_every_shape_runs_with_the_teams_it_is_built_for(cuda_lib):
+    """The registers of a build are shared out over `max_teams` teams, so that many must fit into a CTA's shared memory."""
+    from fp4_all_reduce_b200.parallel.context import launch_plan
+
+    shapes = 0
+    for P in (1, 2, 4, 8):
+        for algo in (0, 1):
+            for inp in (0, 1, 2):
+                for epi in (0, 1, 2, 3):
+                    for width in (3, 6):
+                        teams = int(cuda_lib.fp4ar_has_kernel(P, algo, inp, epi, width))
+                        if teams == 0:
+                            continue
+                        shapes += 1
+                        pl = launch_plan(P, 100000, algo=algo, input=inp, epilogue=epi, team_warps=width)
+                        assert pl["teams"] == teams and pl["team_warps"] == width and not pl["narrow"], (P, algo, inp, epi, width)
+                        assert pl["smem"] <= 227 * 1024
+    assert shapes > 60
+    assert int(cuda_lib.fp4ar_has_kernel(4, 1, 0, 2, 3)) == 4 and int(cuda_lib.fp4ar_has_kernel(8, 1, 0, 2, 3)) == 3
