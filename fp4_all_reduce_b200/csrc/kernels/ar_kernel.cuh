@@ -30,8 +30,9 @@
 //   * Registers bound the six-warp shapes (96 a thread, 18 warps): what spills does not fit the L1 that the
 //     shared memory leaves, and a 12-byte spill in the loop costs 5 - 10 %.  Hence the owner step takes its
 //     sources in batches and addresses are recomputed instead of kept.
-//   * Calls of one or two rows per CTA have a narrow build (MT teams at most, six warps each, up to 168
-//     registers): they are one row's latency, see the rule in runtime.cu.
+//   * Calls of few rows per CTA (up to two, or four where the wide build needs two trips for them as well) have a narrow
+//     build (MT teams at most, six warps each, up to 168 registers): they are a row's or two rows' latency, see the
+//     rule in runtime.cu.
 //   * Every wait is bounded (see fp4ar_async.cuh).
 #pragma once
 #include "../include/fp4ar_codec.cuh"

@@ -29,13 +29,13 @@ static inline ArKernelEntry make_entry() {
   return e;
 }
 
-constexpr int kNarrowTeams = 2;
+constexpr int kNarrowTeams = 2, kNarrowWarps = 6;
 template <int P, int ALGO, int IN>
 static inline void register_narrow(ArKernelEntry* out, int* n) {
-  out[(*n)++] = make_entry<P, ALGO, IN, 0, 6, kNarrowTeams>();
-  out[(*n)++] = make_entry<P, ALGO, IN, 1, 6, kNarrowTeams>();
-  out[(*n)++] = make_entry<P, ALGO, IN, 2, 6, kNarrowTeams>();
-  out[(*n)++] = make_entry<P, ALGO, IN, 3, 6, kNarrowTeams>();
+  out[(*n)++] = make_entry<P, ALGO, IN, 0, kNarrowWarps, kNarrowTeams>();
+  out[(*n)++] = make_entry<P, ALGO, IN, 1, kNarrowWarps, kNarrowTeams>();
+  out[(*n)++] = make_entry<P, ALGO, IN, 2, kNarrowWarps, kNarrowTeams>();
+  out[(*n)++] = make_entry<P, ALGO, IN, 3, kNarrowWarps, kNarrowTeams>();
 }
 
 // Defined once per instantiation unit; each appends its entries.

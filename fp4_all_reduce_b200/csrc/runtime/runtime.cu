@@ -81,14 +81,17 @@ static const ArKernelEntry* find_kernel(int P, int algo, int input, int epi, int
 }
 // Team width: tune[2] of the call if set, else FP4AR_TEAM_WARPS from the environment (a preference: shapes that are
 // not compiled at that width use their default), else the default of the shape.
-static int team_warps_for(const fp4ar_args& a, int nranks, int algo) {
-  if (a.tune[2] > 0) return a.tune[2];
+static int team_warps_from_env() {
   static const int from_env = [] {
     const char* s = std::getenv("FP4AR_TEAM_WARPS");
     const int v = s ? std::atoi(s) : 0;
     return v > 0 ? v : 0;
   }();
-  return from_env > 0 ? from_env : default_team_warps(nranks, algo);
+  return from_env;
+}
+static int team_warps_for(const fp4ar_args& a, int nranks, int algo) {
+  if (a.tune[2] > 0) return a.tune[2];
+  return team_warps_from_env() > 0 ? team_warps_from_env() : default_team_warps(nranks, algo);
 }
 
 #ifdef FP4AR_PHASE_TIMERS
@@ -297,11 +300,12 @@ static int plan_launch(const fp4ar_args& a0, int nranks, int ctas_per_rank, int 
   // Few rows per CTA: the narrow build (six-warp teams, at most two per CTA) where its two teams need no more trips than
   // the teams of the wide one.  A call of that size is one row's latency, and half as many pairs per lane, no spills and
   // every source of an owned row in flight at once shorten it.  Block, BF16 in, one team trip, wide -> narrow: two ranks
-  // 5.2 -> 4.2 us, four 6.6 -> 6.2, eight 9.6 -> 9.2 (NVFP4 in 8.3 -> 7.0).  A call that names a width or a team count
-  // gets what it names.
+  // 6.0 -> 4.5 us, four 6.7 -> 6.6, eight 8.8 -> 7.9 (NVFP4 in 7.8 -> 6.9).  Two trips of each, which is four rows per CTA
+  // where the wide build has three teams (592 rows on 148 SMs): four ranks 13.0 -> 12.5 (NVFP4 out 13.2 -> 12.4), eight
+  // 14.9 -> 13.8.  A call that names a width or a team count gets what it names, an environment that names another width too.
   const int rows_per_cta = (a0.rows + ctas_per_rank - 1) / ctas_per_rank;
-  if (a0.tune[0] <= 0 && a0.tune[2] <= 0 && ke->T == default_team_warps(nranks, algo)) {
-    const ArKernelEntry* ne = find_kernel(nranks, algo, a0.input, a0.epilogue, 6, true);
+  if (a0.tune[0] <= 0 && a0.tune[2] <= 0 && (team_warps_from_env() == 0 || team_warps_from_env() == kNarrowWarps)) {
+    const ArKernelEntry* ne = find_kernel(nranks, algo, a0.input, a0.epilogue, kNarrowWarps, true);
     auto trips = [&](int teams) { return (rows_per_cta + teams - 1) / teams; };
     if (ne && trips(ne->max_teams) <= trips(ke->max_teams)) ke = ne;
   }

@@ -1,5 +1,8 @@
 """CPU tests of the op surface: schemas, fake (meta) implementations, argument validation, window sizes."""
 import ctypes as C
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -184,3 +187,35 @@ def test_every_shape_runs_with_the_teams_it_is_built_for(cuda_lib):
                         assert pl["smem"] <= 227 * 1024
     assert shapes > 60
     assert int(cuda_lib.fp4ar_has_kernel(4, 1, 0, 2, 3)) == 4 and int(cuda_lib.fp4ar_has_kernel(8, 1, 0, 2, 3)) == 3
+
+
+def test_calls_of_few_rows_take_the_narrow_build(cuda_lib):
+    """Two teams of the narrow build need no more trips than the teams of the wide one: up to two rows per CTA, and four where
+    the wide build has three teams.  Whoever names a width or a team count gets it."""
+    from fp4_all_reduce_b200.parallel.context import launch_plan
+
+    for P, wide in ((1, 3), (2, 3), (4, 6), (8, 6)):
+        for rows in (1, 148, 149, 296, 297, 444, 445, 592, 593, 888, 16384):
+            for inp, epi in ((0, 0), (0, 1), (0, 2), (1, 1), (1, 3)):
+                pl = launch_plan(P, rows, input=inp, epilogue=epi)
+                per_cta = -(-rows // 148)
+                narrow = per_cta <= 2 or (P >= 4 and per_cta == 4)
+                assert bool(pl["narrow"]) == narrow and pl["team_warps"] == (6 if narrow else wide), (P, rows, inp, epi, pl)
+                assert pl["teams"] <= per_cta
+                if per_cta <= pl["teams"]:
+                    assert (pl["lag_owner"], pl["lag_finish"]) == (1, 2)
+                assert not launch_plan(P, rows, input=inp, epilogue=epi, team_warps=wide)["narrow"]
+                assert not launch_plan(P, rows, input=inp, epilogue=epi, teams=1)["narrow"]
+
+
+@pytest.mark.parametrize("width", [3, 6])
+def test_a_team_width_from_the_environment_holds_for_calls_of_few_rows(cuda_lib, width):
+    code = """
+from fp4_all_reduce_b200.parallel.context import launch_plan
+print([(p["team_warps"], p["narrow"]) for p in (launch_plan(P, r, epilogue=1) for P in (2, 4) for r in (1, 16384))])
+"""
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, FP4AR_TEAM_WARPS=str(width)), capture_output=True, text=True,
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), timeout=300)
+    assert r.returncode == 0, r.stderr
+    few = (6, 1) if width == 6 else (3, 0)                    # the narrow build is one of six-warp teams
+    assert eval(r.stdout) == [few, (3, 0), few, (width, 0)]   # the wide build of two ranks exists at three warps only
