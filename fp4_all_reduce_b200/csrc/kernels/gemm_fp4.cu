@@ -593,9 +593,13 @@ done:
 // CTA on most of the SMs (N = 6144: 96, 128 or 144 of them), with a short set-up and a short epilogue that stores straight
 // from registers.
 // The K loop is NOT cut over CTAs (a cluster of four that sums its partials takes half as long at K = 8192): the FP32
-// sums are then rounded elsewhere, about one value in 1e5 becomes another E2M1 value, and a step of the largest ones is
-// more than a normalised row may be off by.  Whole chains give the accumulators of the wide tiles bit for bit, so a row
-// does not change with the number of rows that share its call either.
+// sums are then rounded elsewhere and about one value in 1e5 becomes another E2M1 value.  Whole chains give the accumulators
+// of whole wide tiles bit for bit, so a row of such a call does not depend on the rows that share it.  (Above 384 rows it
+// may: tiles that two CTAs share are sums of two chains, which those calls have always had.)
+// Pushed rows leave as one 16-byte and one 2-byte store per 32 columns, straight from registers.  Wider packets cost more than
+// they save where the window is in this GPU's memory (K = 1024, 64 / 200 / 384 rows to four ranks: 7.7 / 8.9 / 9.6 us; one bulk
+// store a row 8.5 / 10.0 / 10.1; neighbouring lanes' stores through shared memory 7.9 / 9.5 / 9.7); over NVLink none of them
+// has been timed.
 // N = 6144, us, 192- and 256-wide tiles -> one block per stage -> now: M = 1: K = 1024 14.3 -> 7.5 -> 6.0, K = 8192 45.3 -> 40.6 -> 30.3;
 // M = 16, K = 2048 14.5 -> 12.4 -> 9.7; K = 8192: M = 64 45.4 -> 40.8 -> 30.7, M = 384 56.1 -> 51.2 -> 49.5;
 // K = 4096: M = 200 27.2 -> 23.3 -> 22.7, M = 384 31.0 -> 26.9 -> 26.2; K = 2048: M = 128 15.0 -> 12.7 -> 10.8, M = 300 16.3 -> 14.0 -> 13.6.

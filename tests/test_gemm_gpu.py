@@ -148,7 +148,8 @@ def test_gemm_reset_keeps_the_kernel_usable():
                                     (33, 512, 256), (100, 64, 512), (5, 192, 1024), (130, 320, 2048)])
 def test_gemm_of_few_rows_equals_the_wide_tiles(M, K, Nn, monkeypatch):
     """Up to 384 rows a CTA takes a narrow tile with its whole K loop: the same chain of MMAs per accumulator as in the
-    256-wide tiles, so sums and rows are the same bit for bit, and the rows equal the host quantiser on those sums."""
+    256-wide tiles that no two CTAs share, so sums and rows are the same bit for bit, and the rows equal the host quantiser on those sums."""
+    assert G.gemm_plan(M, Nn, K, torch.cuda.get_device_properties(0).multi_processor_count)["tile_n"] <= 128
     x, wt = _xw(M, K, Nn, 7)
     gs = G.calibrate_gs(x, wt)
     q, acc = G.gemm_nvfp4(x, wt, gs, want_acc=True)

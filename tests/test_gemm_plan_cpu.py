@@ -51,6 +51,22 @@ def test_schedule_covers_every_k_block_once(M, K, sms):
         assert max(cut) - min(cut) <= 1
 
 
+@pytest.mark.parametrize("M,width,tiles", [(1, 64, 96), (64, 64, 96), (128, 64, 96), (129, 96, 128), (256, 96, 128), (257, 128, 144), (384, 128, 144)])
+@pytest.mark.parametrize("K", [64, 2048, 8192])
+def test_few_rows_take_narrow_tiles_with_whole_k_loops(M, width, tiles, K):
+    pl = G.gemm_plan(M, 6144, K)
+    assert pl == {"pair": 0, "tile_n": width, "stream_k": 0, "units": tiles, "tiles": tiles}
+
+
+def test_where_the_narrow_tiles_end():
+    """Tiles of 64, 96 and 128 columns are the few-row kernel's, 192 and 256 those of the wide ones."""
+    assert G.gemm_plan(385, 6144, 2048)["tile_n"] >= 192 and G.gemm_plan(1024, 6144, 8192)["tile_n"] >= 192
+    assert G.gemm_plan(1, 256, 64) == {"pair": 0, "tile_n": 64, "stream_k": 0, "units": 4, "tiles": 4}
+    assert G.gemm_plan(1, 12288, 2048)["tile_n"] == 96
+    assert G.gemm_plan(1, 24576, 2048)["tile_n"] >= 192        # more tiles of every narrow width than SMs
+    assert G.gemm_plan(300, 6144, 2048, sms=132)["tile_n"] >= 192
+
+
 def test_shape_choice_for_the_bench_shapes():
     assert G.gemm_plan(4096, 6144, 8192)["pair"] == 1 and G.gemm_plan(4096, 6144, 8192)["stream_k"] == 1
     assert G.gemm_plan(16384, 6144, 8192)["stream_k"] == 0            # 1536 pair tiles on 74 pairs: 20.8 waves
