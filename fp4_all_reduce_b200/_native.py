@@ -153,9 +153,7 @@ def front():
     import importlib.machinery
     import importlib.util
 
-    path = _build.front_path()
-    if not path.exists():
-        raise RuntimeError(f"{path} is missing: build it with `python -m fp4_all_reduce_b200.build` (needs g++; no GPU required)")
+    path = _build.check_front()
     import torch  # noqa: F401  (the module links against its libraries)
 
     cuda()

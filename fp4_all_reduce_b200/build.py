@@ -10,7 +10,8 @@ produces, next to this file,
 
     lib/libfp4ar.so         CUDA kernels + host runtime for sm_100a (nvcc, cross-compiles without a GPU)
     lib/libfp4ar_oracle.so  the host-only bit-exact model (g++)
-    lib/_fp4ar_front.so     the torch front end: checks, output allocation and launch of one call in C++ (g++, torch headers)
+    lib/_fp4ar_front.so     the torch front end: checks, output allocation and launch of one call in C++ (g++, torch headers);
+                            left out where there is no torch: the other two need none
 
 Each translation unit is compiled separately and in parallel; an object is rebuilt when its source or
 any header under csrc/ changed.  ptxas resource usage of every kernel is appended to
@@ -136,6 +137,27 @@ def front_path() -> Path:
     return LIB / "_fp4ar_front.so"
 
 
+def _front_target() -> str:
+    """What a front end is built for: it runs in this interpreter with this torch and no other."""
+    import sysconfig
+
+    import torch
+
+    return f"torch {torch.__version__}, python {sysconfig.get_python_version()}"
+
+
+def check_front() -> Path:
+    """The front end's path, if there is one; not one that was built for another interpreter or torch than those that ask."""
+    path, target = front_path(), LIB / "front.target"
+    if not path.exists():
+        raise RuntimeError(f"{path} is missing: build it with `python -m fp4_all_reduce_b200.build` (needs g++; no GPU required)")
+    built = target.read_text() if target.exists() else _front_target()      # a library brought here by itself is taken as it is
+    if built != _front_target():
+        raise RuntimeError(f"{path} was built for {built}, this is {_front_target()}: build it again with "
+                           "`python -m fp4_all_reduce_b200.build`")
+    return path
+
+
 def build_front(force: bool = False, verbose: bool = False) -> Path:
     """The torch front end, an extension module of this interpreter against the installed torch's headers."""
     import sysconfig
@@ -153,12 +175,13 @@ def build_front(force: bool = False, verbose: bool = False) -> Path:
            "-ltorch_cuda", "-ltorch_python"]
     stamp_file = LIB / "front.stamp"
     stamp = _stamp(src, _headers_digest() + torch.__version__ + sysconfig.get_python_version() + " ".join(cmd))
-    if not force and out.exists() and stamp_file.exists() and stamp_file.read_text() == stamp:
+    if not force and out.exists() and stamp_file.exists() and stamp_file.read_text() == stamp and (LIB / "front.target").exists():
         return out
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed:\n{r.stdout}\n{r.stderr}")
     stamp_file.write_text(stamp)
+    (LIB / "front.target").write_text(_front_target())
     if verbose:
         print("[build] torch_front.cpp")
     return out
@@ -222,9 +245,14 @@ def resources(log: Path | None = None) -> list[dict]:
 
 
 def build_all(force: bool = False, verbose: bool = False) -> dict[str, Path]:
+    import importlib.util
+
     with cf.ThreadPoolExecutor(max_workers=1) as ex:
-        front = ex.submit(build_front, force, verbose)
+        front = ex.submit(build_front, force, verbose) if importlib.util.find_spec("torch") else None
         libs = {"oracle": build_oracle(force, verbose), "cuda": build_cuda(force, verbose)}
+        if front is None:
+            print("[build] no torch: the front end is left out")
+            return libs
         return {**libs, "front": front.result()}
 
 

@@ -1,6 +1,8 @@
 """Source manifest (provenance) and the ptxas resource parser of the build script, on the host."""
 from pathlib import Path
 
+import pytest
+
 from fp4_all_reduce_b200 import build as B
 
 
@@ -40,3 +42,27 @@ def test_resource_log_parser(tmp_path):
     rs = B.resources(log)
     assert rs == [{"symbol": "_Z1kv", "stack": 40, "spill_stores": 4, "spill_loads": 12, "registers": 168},
                   {"symbol": "_Z1jv", "stack": 0, "spill_stores": 0, "spill_loads": 0, "registers": 32}]
+
+
+def test_c_library_builds_without_torch(monkeypatch, capsys):
+    import importlib.util
+
+    find = importlib.util.find_spec
+    monkeypatch.setattr(importlib.util, "find_spec", lambda name, *a: None if name == "torch" else find(name, *a))
+    monkeypatch.setattr(B, "build_oracle", lambda *a: "oracle")
+    monkeypatch.setattr(B, "build_cuda", lambda *a: "cuda")
+    monkeypatch.setattr(B, "build_front", lambda *a: pytest.fail("needs torch"))
+    assert B.build_all() == {"oracle": "oracle", "cuda": "cuda"} and "left out" in capsys.readouterr().out
+
+
+def test_front_end_of_another_torch_is_refused(tmp_path, monkeypatch):
+    monkeypatch.setattr(B, "LIB", tmp_path)
+    with pytest.raises(RuntimeError, match="is missing"):
+        B.check_front()
+    B.front_path().write_bytes(b"")
+    assert B.check_front() == B.front_path()
+    (tmp_path / "front.target").write_text("torch 1.0, python 3.12")
+    with pytest.raises(RuntimeError, match="built for torch 1.0"):
+        B.check_front()
+    (tmp_path / "front.target").write_text(B._front_target())
+    assert B.check_front() == B.front_path()
