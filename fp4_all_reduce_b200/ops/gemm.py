@@ -34,6 +34,12 @@ def _check(x: torch.Tensor, wt: torch.Tensor):
     return M, Nn, K
 
 
+def _holds(t: torch.Tensor, nbytes: int, device, name: str) -> None:
+    """The kernels trust their pointers: `t` is `nbytes` of contiguous memory of `device` at least."""
+    if t.device != device or not t.is_contiguous() or t.nbytes < nbytes:
+        raise ValueError(f"{name} must be contiguous, on {device} and hold {nbytes} bytes")
+
+
 def calibrate_gs(x: torch.Tensor, wt: torch.Tensor) -> float:
     """Static scale of this rank's partial from a calibration batch (runs a plain BF16 matmul)."""
     y = torch.matmul(x, wt.t()).float()
@@ -51,6 +57,10 @@ def gemm_push(ctx, x: torch.Tensor, wt: torch.Tensor, gs_self: float, *, two_sho
     M, Nn, K = _check(x, wt)
     if Nn != N.HIDDEN:
         raise ValueError("the AllReduce windows are laid out for N = 6144")
+    if x.device != ctx.device or wt.device != ctx.device:
+        raise ValueError(f"x and wt must be on the context's device {ctx.device}")
+    if local_q is not None:
+        _holds(local_q, M * N.QROW_BYTES, x.device, "local_q")
     view = ctx.push_view(local_rank)
     if two_shot is None:
         two_shot = ctx.nranks > 2
@@ -69,13 +79,22 @@ def gemm_all_reduce_add_rms_norm(ctx, x: torch.Tensor, wt: torch.Tensor, gs: Seq
 
     M = x.shape[0]
     two_shot = ctx.nranks > 2
+    # everything is checked before the push: rows in the windows that no launch takes would spoil the next call
+    if epilogue not in (N.EPI_NORM_BF16, N.EPI_NORM_NVFP4, N.EPI_NORM_MXFP8):
+        raise ValueError("epilogue must be 1 (BF16), 2 (NVFP4) or 3 (MXFP8)")
+    if len(gs) < ctx.nranks or not all(float(g) > 0.0 for g in gs[:ctx.nranks]):
+        raise ValueError(f"gs must hold one positive static scale per rank ({ctx.nranks})")
+    _holds(residual, M * 2 * N.HIDDEN, ctx.device, "residual")
+    _holds(weight, 2 * N.HIDDEN, ctx.device, "weight")
+    row_bytes = {N.EPI_NORM_BF16: 2 * N.HIDDEN, N.EPI_NORM_NVFP4: N.QROW_BYTES, N.EPI_NORM_MXFP8: N.MXROW_BYTES}[epilogue]
+    if out is not None:
+        _holds(out, M * row_bytes, ctx.device, "out")
     gemm_push(ctx, x, wt, float(gs[ctx.rank]), two_shot=two_shot)
     o = q = None
     if epilogue == N.EPI_NORM_BF16:
         o = out if out is not None else torch.empty(M, N.HIDDEN, dtype=torch.bfloat16, device=x.device)
     else:
-        nb = N.QROW_BYTES if epilogue == N.EPI_NORM_NVFP4 else N.MXROW_BYTES
-        q = out if out is not None else torch.empty(M, nb, dtype=torch.uint8, device=x.device)
+        q = out if out is not None else torch.empty(M, row_bytes, dtype=torch.uint8, device=x.device)
     ctx.launch(make_args(x=None, out=o, rows=M, input=N.IN_PUSHED, gs=list(gs), epilogue=epilogue, res_in=residual,
                          res_out=residual, weight=weight, eps=eps, weight_bias=weight_bias, outq=q, qscale=qscale,
                          algo=N.ALGO_TWOSHOT if two_shot else N.ALGO_ONESHOT))

@@ -96,3 +96,22 @@ def test_a_number_beyond_a_double_is_an_overflow():
     with pytest.raises(OverflowError):
         ctx.all_reduce_add_rms_norm(_bf16(), _bf16(), _bf16(1).view(-1), eps=10**400, mode=N.MODE_COMPUTE)
     ctx.close()
+
+
+def test_fused_linear_checks_everything_before_it_pushes():
+    """A refused call leaves the windows as they were: nothing was pushed that no launch would take."""
+    ctx = SoloRankContext(2, ROWS)
+    x, wt, res, w = _bf16(ROWS, 128), _bf16(N.HIDDEN, 128), _bf16(), _bf16(1).view(-1)
+    window = ctx.window.clone()
+    q8 = torch.zeros(ROWS, N.QROW_BYTES, dtype=torch.uint8, device="cuda")
+    good = dict(x=x, wt=wt, gs=[1.0, 1.0], residual=res, weight=w)
+    for bad in (dict(residual=res[:ROWS - 1]), dict(residual=res.cpu()), dict(weight=w[:64]), dict(weight=w.cpu()), dict(out=_bf16(ROWS - 1)),
+                dict(epilogue=2, out=q8[:ROWS - 1]), dict(epilogue=3, out=q8), dict(epilogue=0), dict(gs=[1.0]), dict(gs=[1.0, 0.0]),
+                dict(x=x.cpu()), dict(wt=_bf16(256, 128))):
+        with pytest.raises(ValueError):
+            G.gemm_all_reduce_add_rms_norm(ctx, **{**good, **bad})
+    with pytest.raises(ValueError, match="local_q"):
+        G.gemm_push(ctx, x, wt, 1.0, local_q=q8[:ROWS - 1])
+    torch.cuda.synchronize()
+    assert torch.equal(ctx.window, window)
+    ctx.close()
