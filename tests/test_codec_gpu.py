@@ -45,6 +45,23 @@ def test_encode_static_bit_exact():
     assert np.count_nonzero(q.cpu().numpy() != O.encode_static(O.bf16_bits(x), gs)) == 0
 
 
+@pytest.mark.parametrize("rows", [592, 593, 1333])
+def test_calls_of_several_trips_bit_exact(rows):
+    """More rows than the 592 teams of the encoder and of the sum on 148 SMs: their second and third rows."""
+    x = D.partial(rows, 4)
+    bits = O.bf16_bits(x)
+    assert np.array_equal(codec.encode_static(x.to(DEV), 0.05).cpu().numpy(), O.encode_static(bits, 0.05))
+    q, rs = codec.encode(x.to(DEV))
+    v, s, r = O.encode(bits)
+    assert np.array_equal(q.cpu().numpy()[:, :3072], v) and np.array_equal(q.cpu().numpy()[:, 3072:], s)
+    assert np.array_equal(rs.cpu().numpy().view(np.uint32), r.view(np.uint32))
+    for n in (1, 3, 8):
+        xs = [x] + [D.partial(rows, 40 + i) for i in range(n - 1)]
+        enc = [codec.encode(t.to(DEV)) for t in xs]
+        out = codec.decode_sum([e[0] for e in enc], [e[1] for e in enc])
+        assert _same_bf16(out, O.allreduce([O.bf16_bits(t) for t in xs], algo=0)["out"]) == 0
+
+
 @pytest.mark.parametrize("P", [1, 2, 4, 8])
 def test_decode_sum_bit_exact(P):
     rows = 200

@@ -115,3 +115,60 @@ def test_fused_linear_checks_everything_before_it_pushes():
     torch.cuda.synchronize()
     assert torch.equal(ctx.window, window)
     ctx.close()
+
+
+def test_context_calls_name_what_is_wrong():
+    """What the native front end does not take falls to the wrapper's checks, on CUDA tensors as well."""
+    ctx = SoloRankContext(2, ROWS)
+    x, res, w = _bf16(), _bf16(), _bf16(1).view(-1)
+    q, rs = codec.encode(x + 1)
+    kw = dict(mode=N.MODE_COMPUTE)
+
+    def refused(match, fn, *a, **k):
+        with pytest.raises(ValueError, match=match):
+            fn(*a, **{**kw, **k})
+
+    ar, block = ctx.all_reduce, ctx.all_reduce_add_rms_norm
+    refused("must be bfloat16", ar, x.float())
+    refused("shape", ar, _bf16(ROWS, 3072))
+    refused("contiguous", ar, _bf16(ROWS, 2 * N.HIDDEN)[:, ::2])
+    refused("is on cpu", ar, x.cpu())
+    refused("max_rows", ar, _bf16(ROWS + 1))
+    refused("out must have 8 rows", ar, x, _bf16(ROWS + 1))
+    refused("out must be", ar, x, q)
+    refused("out is on cpu", ar, x, _bf16(device="cpu"))
+    for gs in (None, [1.0], [1.0, 0.0], [1.0, -1.0], [1.0, float("nan")]):
+        refused("gs", ar, q, gs=gs)
+    refused("residual must have 8 rows", block, x, res[:4], w)
+    refused("residual is on cpu", block, x, res.cpu(), w)
+    refused("residual_out", block, x, res, w, residual_out=_bf16(ROWS, 3072))
+    refused("weight", block, x, res, w.float())
+    refused("weight", block, x, res, _bf16(2).view(-1)[::2])
+    refused("epilogue", block, x, res, w, epilogue=0)
+    refused("out must be", block, x, res, w, epilogue=2, out=x)
+    refused("out must have shape", block, x, res, w, epilogue=3, out=q)
+    refused("mode=MODE_COMPUTE", ar, x, mode=N.MODE_FUSED)
+    assert ctx.status().ok
+    ctx.close()
+
+
+def test_unusual_but_valid_context_calls_equal_the_plain_one():
+    import numpy as np
+
+    ctx = SoloRankContext(2, ROWS)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(ROWS, N.HIDDEN, generator=g, device="cuda").to(torch.bfloat16)
+    res, w = x + 1, torch.randn(N.HIDDEN, generator=g, device="cuda").to(torch.bfloat16)
+    q = codec.encode_static(x, 0.01)
+    plain = ctx.all_reduce(q, gs=[0.01, 0.01], mode=N.MODE_COMPUTE)
+    for gs in ((0.01, 0.01), np.array([0.01, 0.01]), torch.tensor([0.01, 0.01]), [np.float32(0.01), torch.tensor(0.01)]):
+        assert torch.equal(ctx.all_reduce(q, gs=gs, mode=N.MODE_COMPUTE), plain)
+    y, r = ctx.all_reduce_add_rms_norm(x, res.clone(), w, mode=N.MODE_COMPUTE)
+    weight = torch.nn.Parameter(w.view(1, -1))
+    out, res_out = torch.empty_like(x), torch.empty_like(x)
+    kept = res.clone()
+    y2, r2 = ctx.all_reduce_add_rms_norm(x, kept, weight, eps=np.float64(1e-6), weight_bias=1, out=out, residual_out=res_out, mode=N.MODE_COMPUTE)
+    assert y2 is out and r2 is res_out and torch.equal(kept, res) and torch.equal(y, y2) and torch.equal(r, r2)
+    empty = ctx.all_reduce(x[:0], mode=N.MODE_COMPUTE)
+    assert empty.shape == (0, N.HIDDEN)
+    ctx.close()
