@@ -77,3 +77,25 @@ def test_oversized_call_is_rejected_on_the_host():
     a.hidden = 4096
     assert lib.fp4ar_launch(ctx, (N.Args * 1)(a), None) == 1
     lib.fp4ar_destroy(ctx)
+
+
+@pytest.mark.parametrize("nranks", [2, 4, 8])
+def test_missing_peer_ends_a_block_of_many_rows(nranks):
+    """Input and residual rows are on their way into shared memory when the wait for the peer gives up: the CTA lets them land,
+    reports and ends, and after a reset of the context its memory serves other calls as before."""
+    rows = 2000
+    lib, ctx, wins = _lonely_rank0(nranks, rows)
+    N.check(lib.fp4ar_set_timeout_ms(ctx, 20), "timeout")
+    x, res, w = D.partial(rows, 0).cuda(), D.residual(rows).cuda(), D.norm_weight().cuda()
+    out = torch.zeros_like(x)
+    t0 = time.time()
+    N.check(lib.fp4ar_launch(ctx, (N.Args * 1)(make_args(x=x, out=out, rows=rows, epilogue=1, res_in=res, res_out=res, weight=w)), None), "launch")
+    torch.cuda.synchronize()
+    assert time.time() - t0 < 5.0
+    st = N.StatusWords()
+    N.check(lib.fp4ar_status(ctx, 0, C.byref(st)), "status")
+    assert st.code == 1 and st.source != 0
+    N.check(lib.fp4ar_reset(ctx), "reset")
+    lib.fp4ar_destroy(ctx)
+    rec = gate_cell_emulated(CellConfig(nranks=nranks, rows=300, epilogue=1), reps=3, graph_calls=0)
+    assert rec["pass"], rec
