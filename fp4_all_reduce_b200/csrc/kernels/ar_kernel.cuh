@@ -26,10 +26,11 @@
 //     bulk store each.  (The residual used to go global -> registers -> global in 16-byte pieces at a
 //     64-byte stride, and its loads were issued where they were needed: finishing a row took 5000 - 6700
 //     cycles instead of 1250 without the epilogue.  16384 rows, BF16, one rank's work: two ranks 157 -> 145 us
-//     per block, four 198 -> 168, eight 232 -> 175 with the spills below gone; 123 us at the copy rate.)
+//     per block, four 198 -> 168, eight 232 -> 175 with most of the spills below gone; 123 us at the copy rate.)
 //   * Registers bound the six-warp shapes (96 a thread, 18 warps): what spills does not fit the L1 that the
 //     shared memory leaves, and a 12-byte spill in the loop costs 5 - 10 %.  Hence the owner step takes its
-//     sources in batches and addresses are recomputed instead of kept.
+//     sources in batches and addresses are recomputed instead of kept.  (What is left are 4 - 12 bytes in the
+//     eight-rank shapes.)
 //   * Calls of few rows per CTA (up to two, or four where the wide build needs two trips for them as well) have a narrow
 //     build (MT teams at most, six warps each, up to 168 registers): they are a row's or two rows' latency, see the
 //     rule in runtime.cu.
@@ -464,8 +465,8 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T, MT>::kMa
         const int row = row_of(ko);
         uint8_t* rec_own = recs + (ko % NREC) * kRecStride;
         // Every rank's contribution in rank order, kOwnBatch ranks at a time: the loads of a batch are issued together,
-        // and where some have not arrived all of those are asked for again
-        // together, one round trip for all instead of one each.  The own contribution comes from the record ring.
+        // and where some have not arrived those are asked for again together, one round trip for all instead of one
+        // each.  The own contribution comes from the record ring.
         constexpr int kOwnBatch = MT > 0 ? P : (P == 4 ? 4 : 2);
         char* const src0 = my_buf() + rs_slot(0, row);
         auto own_src = [&](int src) { return src0 + (size_t)src * prm.rs_stride; };

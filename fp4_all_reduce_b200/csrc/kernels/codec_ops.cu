@@ -98,9 +98,9 @@ __device__ __forceinline__ void decode_acc_natural(float* acc, uint4 q, uint32_t
 // ---------------------------------------------------------------------------------------------
 // Bound by memory, if enough of it is in flight all the time: a team loads its next row before it works on the one at hand
 // (two rows at once per trip left the memory idle while both were encoded, and their coarse trips left SMs idle at a few
-// thousand rows).  The loads are evict-first, so that the rows written stay in the L2 for whoever reads them.
-// Back-to-back calls: 8192 rows 26.7 -> 18.5 us (0.94 of the copy rate counted without the write-back of the rows), 16384
-// rows 47.5 -> 35.0, with a static scale 36.8 -> 33.6; 2048 rows 9.3 -> 7.7 on the device.
+// thousand rows).  Loads and value stores are evict-first.  Back-to-back calls over fresh inputs: 8192 rows 27.2 -> 23.1 us
+// (129 MB read and written, 0.85 of the copy rate of 6546 GB/s), 16384 rows 50.3 -> 43.7, 2048 rows 9.4 -> 7.8; with a static scale,
+// which needs no exchange between the warps, 23.0 -> 22.8, 43.1 -> 43.1 and 7.8 -> 7.3.
 constexpr int kEncodeTeamsPerSm = 4;
 template <bool STATIC>
 __global__ void __launch_bounds__(kTeamThreads, kEncodeTeamsPerSm)
@@ -165,9 +165,9 @@ __host__ __device__ constexpr int decode_rows_per_trip(int ns, bool reenc) {
 constexpr int kDecodeTeamsPerSm = 4;
 
 // The owner step works long enough on a row for the memory to idle meanwhile, so it loads its next row once the sum is in
-// the accumulators, for up to four sources, where the registers allow it (9000 rows, two sources 46.2 -> 41.0 us; 4096 rows,
-// four 28.0 -> 27.7; eight spill and lose, 41.0 -> 45.6).  The plain sum gains nothing by it (16384 rows, one source 45.7 either way;
-// 3001 rows, four 14.7 -> 15.7).
+// the accumulators, for up to four sources (9000 rows, two sources 46.4 -> 38.1 us; four sources, which spill 8 bytes for it,
+// 4096 rows 28.2 -> 27.2 and 16384 rows 99.5 -> 95.3; eight spill more and lose, 39.9 -> 45.1 and 147.7 -> 161.2).  The plain sum gains
+// nothing by it (16384 rows, one source 45.9 -> 46.2, eight 111 -> 125; 3001 rows, four 15.3 -> 17.0).
 __host__ __device__ constexpr bool decode_loads_ahead(int ns, bool reenc) { return reenc && ns <= 4; }
 
 template <int NS, bool REENC>
@@ -249,8 +249,9 @@ decode_sum_kernel(SrcList src, long pitch, int rows, char* rec_out, char* out) {
 // The sum of squares follows the fixed tree of the host model: per pair (t0 + t1) + (t2 + t3) over its four
 // chunk sums, a butterfly over the 32 pairs of a group (= one warp here), then the six groups in order.
 // Quantised outputs cost enough work per row that the memory idles during it: those shapes load a row ahead, with the
-// weights in shared memory to have the registers for it (16384 rows: NVFP4 out 118.5 -> 107.5 us, MXFP8 121.8 -> 116.6; 3000
-// rows, NVFP4 24.1 -> 21.7).  BF16 out runs at the copy rate as it is and loses by it (124.9 -> 139.7 us).
+// weights in shared memory to have the registers for it (NVFP4 out: 16384 rows 119.0 -> 109.5 us, 3000 rows 25.1 -> 22.1; MXFP8:
+// 3000 rows 25.5 -> 23.4, 16384 rows 118.9 -> 119.9).  BF16 out runs at the copy rate as it is and loses by it (16384 rows
+// 125.9 -> 144.8).
 // ---------------------------------------------------------------------------------------------
 __host__ __device__ constexpr bool norm_loads_ahead(int epi) { return epi >= 2; }
 template <int EPI>

@@ -600,9 +600,9 @@ done:
 // they save where the window is in this GPU's memory (K = 1024, 64 / 200 / 384 rows to four ranks: 7.7 / 8.9 / 9.6 us; one bulk
 // store a row 8.5 / 10.0 / 10.1; neighbouring lanes' stores through shared memory 7.9 / 9.5 / 9.7); over NVLink none of them
 // has been timed.
-// N = 6144, us, 192- and 256-wide tiles -> one block per stage -> now: M = 1: K = 1024 14.3 -> 7.5 -> 6.0, K = 8192 45.3 -> 40.6 -> 30.3;
-// M = 16, K = 2048 14.5 -> 12.4 -> 9.7; K = 8192: M = 64 45.4 -> 40.8 -> 30.7, M = 384 56.1 -> 51.2 -> 49.5;
-// K = 4096: M = 200 27.2 -> 23.3 -> 22.7, M = 384 31.0 -> 26.9 -> 26.2; K = 2048: M = 128 15.0 -> 12.7 -> 10.8, M = 300 16.3 -> 14.0 -> 13.6.
+// N = 6144, fresh weights for every call, us, 192- and 256-wide tiles -> these: M = 1: K = 1024 9.8 -> 7.2, K = 8192 48.6 -> 30.3;
+// M = 64: K = 1024 10.6 -> 7.3, K = 2048 15.2 -> 10.7, K = 8192 44.4 -> 30.5; M = 128, K = 2048 15.3 -> 11.9; M = 200, K = 4096 26.7 -> 21.5;
+// M = 300, K = 2048 16.5 -> 13.5; M = 384: K = 1024 11.6 -> 8.9, K = 4096 29.6 -> 22.5, K = 8192 48.9 -> 42.4.
 // The A box holds only the valid rows, rounded up to eight: the MMA still takes 128 rows, and what it reads for the rest
 // is the start of the B block or whatever follows it in shared memory, whose products land in accumulator rows that nobody
 // reads.
@@ -1105,7 +1105,7 @@ extern "C" int fp4ar_gemm_nvfp4(const fp4ar_push_view* push, int two_shot, const
   CUtensorMap ma, mb;
   if (pl.narrow) {
     p.a_rows = M < kBM ? (M + 7) / 8 * 8 : kBM;
-    // K blocks per stage: as many, up to four, as leave the ring two stages (M = 64, K = 8192: 30.7 us, with four shorter stages 38.1)
+    // K blocks per stage: as many, up to four, as leave the ring two stages (M = 64, K = 8192: 30.5 us; four shorter stages took 38)
     p.atoms = 4;
     while (p.atoms > 1 && (p.atoms > K / kBK || p.atoms * (p.a_rows + bn) * kBK * 2 > 100 * 1024)) p.atoms /= 2;
     const bool maps = p.atoms > 1 ? make_map_3d(&ma, x, M, K, p.a_rows, p.atoms) && make_map_3d(&mb, wt, N, K, bn, p.atoms)
