@@ -78,13 +78,15 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
                : "=r"(done) : "r"(smem_addr(bar)), "r"(parity) : "memory");
   return done != 0;
 }
-// Wait for a local bulk load.  Returns false (after reporting) when the limit ran out or the CTA aborted.
+// Wait for a local bulk load.  Returns false (after reporting) when the limit ran out or the CTA aborted, but not before 256
+// tests: a load lands in its CTA's shared memory whether anybody wants it or not, so an aborting CTA gives every one it has
+// issued that long.  (A wait by the clock there, or at the kernel's end, costs the eight-rank shapes registers and 1 - 2 %.)
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, const WaitCtx& w, uint32_t row) {
   if (mbar_test(bar, parity)) return true;
   const unsigned long long t0 = global_timer_ns();
   uint32_t n = 0;
   while (!mbar_test(bar, parity)) {
-    if ((++n & 63u) == 0u) {
+    if ((++n & 255u) == 0u) {
       if (*w.cta_abort) return false;
       if (global_timer_ns() - t0 > w.limit_ns) { report_wait_failure(w, kStatusLoadTimeout, row, 0, 4); return false; }
     }

@@ -850,10 +850,6 @@ __global__ void __launch_bounds__(32 * T * ArShape<P, ALGO, IN, EPI, T, MT>::kMa
 
   if (kTwoShot ? lane == 0 : leader) bulk_wait_done<0>();
   __syncthreads();
-  // Waits of a CTA that gave up return at once, those for its own loads too: 2 ms for what is still on its way into its
-  // shared memory.  (Waiting longer in those waits instead cost eight ranks with NVFP4 input 2 % in registers.)
-  if (*abort_flag != 0u)
-    for (int i = 0; i < 2000; i++) __nanosleep(1000);
   if (threadIdx.x == 0) io.ctrl[cta] = call + 1u;
 }
 
