@@ -99,7 +99,7 @@ __device__ __forceinline__ void decode_acc_natural(float* acc, uint4 q, uint32_t
 // Bound by memory, if enough of it is in flight all the time: a team loads its next row before it works on the one at hand
 // (two rows at once per trip left the memory idle while both were encoded, and their coarse trips left SMs idle at a few
 // thousand rows).  Loads and value stores are evict-first.  Back-to-back calls over fresh inputs: 8192 rows 27.2 -> 23.1 us
-// (129 MB read and written, 0.85 of the copy rate of 6546 GB/s), 16384 rows 50.3 -> 43.7, 2048 rows 9.4 -> 7.8; with a static scale,
+// (129 MB read and written at 5.6 TB/s), 16384 rows 50.3 -> 43.7, 2048 rows 9.4 -> 7.8; with a static scale,
 // which needs no exchange between the warps, 23.0 -> 22.8, 43.1 -> 43.1 and 7.8 -> 7.3.
 constexpr int kEncodeTeamsPerSm = 4;
 template <bool STATIC>

@@ -377,17 +377,15 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      uint32_t it = 0;
       SegIter seg(p.stream_k, tiles, kblocks, unit, units);
       Seg sg;
       while (seg.next(sg)) {
         int m0, n0;
         tile_coords<BN, G>(sg.tile, m_tiles, n_tiles, m0, n0);
-        for (int j = 0; j < sg.count; j++, it++) {
+        for (int j = 0; j < sg.count; j++, issued++) {
           const int kb = sg.lo + j;
-          const int s = it % kStages;
-          if (!gemm_wait(empty + s, ((it / kStages) & 1u) ^ 1u, gw, 1)) goto done;
-          issued = it + 1;
+          const int s = issued % kStages;
+          if (!gemm_wait(empty + s, ((issued / kStages) & 1u) ^ 1u, gw, 1)) goto done;
           if constexpr (G == 2) {
             // both CTAs' bytes are counted under the leader's barrier; only the leader announces them
             const uint32_t lead_full = cluster_addr(full + s, 0u);
@@ -651,16 +649,15 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 
   if (warp == 0) {
     if (lane == 0) {
-      for (int it = 0, st = 0, round = 0; it < trips; it++) {
+      for (int st = 0, round = 0; issued < trips; issued++) {
         if (!gemm_wait(empty + st, (round & 1u) ^ 1u, gw, 1)) break;
-        issued = it + 1;
         mbar_arrive_expect(full + st, stage_bytes);
         if (atoms > 1) {
-          tma_load_3d(ring + st * stage_bytes, &map_a, m0, it * atoms, full + st);
-          tma_load_3d(ring + st * stage_bytes + a_bytes, &map_b, n0, it * atoms, full + st);
+          tma_load_3d(ring + st * stage_bytes, &map_a, m0, issued * atoms, full + st);
+          tma_load_3d(ring + st * stage_bytes + a_bytes, &map_b, n0, issued * atoms, full + st);
         } else {
-          tma_load_2d(ring + st * stage_bytes, &map_a, it * kBK, m0, full + st);
-          tma_load_2d(ring + st * stage_bytes + a_bytes, &map_b, it * kBK, n0, full + st);
+          tma_load_2d(ring + st * stage_bytes, &map_a, issued * kBK, m0, full + st);
+          tma_load_2d(ring + st * stage_bytes + a_bytes, &map_b, issued * kBK, n0, full + st);
         }
         if (++st == stages) { st = 0; round++; }
       }
