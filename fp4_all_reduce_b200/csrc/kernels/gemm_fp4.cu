@@ -1147,14 +1147,13 @@ extern "C" int fp4ar_gemm_reset(void) {
   std::lock_guard<std::mutex> g(g_stream_k_mu);
   if (cudaDeviceSynchronize() != cudaSuccess) return cuda_fail();     // what was enqueued before the lock was taken
   StreamKPool& pool = g_stream_k[dev];
+  auto in_use = [](const StreamKSpace& s) { return s.graph_owned && !s.idle.load(std::memory_order_acquire); };
+  for (auto& s : pool.spaces)
+    if (in_use(*s) && cudaMemset((char*)s->mem + stream_k_partial_bytes(), 0, stream_k_flag_bytes()) != cudaSuccess) return cuda_fail();
   std::vector<std::unique_ptr<StreamKSpace>> kept;
   for (auto& s : pool.spaces) {
-    if (s->graph_owned && !s->idle.load(std::memory_order_acquire)) {
-      if (cudaMemset((char*)s->mem + stream_k_partial_bytes(), 0, stream_k_flag_bytes()) != cudaSuccess) return cuda_fail();
-      kept.push_back(std::move(s));
-    } else {
-      cudaFree(s->mem);
-    }
+    if (in_use(*s)) kept.push_back(std::move(s));
+    else cudaFree(s->mem);
   }
   pool.spaces.swap(kept);
   if (pool.shared) { cudaFree(pool.shared->mem); pool.shared.reset(); }
